@@ -166,8 +166,8 @@ __global__ void sell_gather_k(int64_t slots, const int32_t* __restrict__ map,
 
 // ---------------------------------------------------------------------------
 // Deterministic multi-dot: out[k] = sum_i V[k][i] * w[i] for k < nv.
-// Stage 1 writes per-block partials (fixed grid); stage 2 sums them in a
-// fixed tree order.
+// Every block writes its partial sums (fixed grid); the last one to finish
+// sums them in a fixed tree order.
 //
 // FP32 vectors: every product is formed exactly (p + e with e = fma(a, b,
 // -p)) and accumulated as a two-float sum (Knuth two-sum); warp reductions
@@ -183,11 +183,6 @@ __device__ __forceinline__ void two_sum_acc(float& s, float& c, float x) {
   c += (s - (t - bp)) + (x - bp);
   s = t;
 }
-__device__ __forceinline__ void acc_prod(double a, double b, double& s,
-                                         double& c) {
-  s = fma(a, b, s);
-  (void)c;
-}
 __device__ __forceinline__ void acc_prod(float a, float b, float& s,
                                          float& c) {
   const float p = a * b;
@@ -195,12 +190,6 @@ __device__ __forceinline__ void acc_prod(float a, float b, float& s,
   two_sum_acc(s, c, p);
 }
 // warp sum of (s, c); result valid in lane 0 as a double
-__device__ __forceinline__ double warp_sum(double s, double c) {
-  double v = s + c;
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
-  return v;
-}
 __device__ __forceinline__ double warp_sum(float s, float c) {
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) {
@@ -212,57 +201,193 @@ __device__ __forceinline__ double warp_sum(float s, float c) {
   return double(s) + double(c);
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kBlock)
-    mdot_k(int64_t n, int nv, const T* __restrict__ V, int64_t ld,
-           const T* __restrict__ w, double* __restrict__ partial) {
-  __shared__ double red[kTile][kBlock / 32];
-  const int G = gridDim.x;
-  const int64_t stride = int64_t(G) * blockDim.x;
+// Final sums of a reduction in the kernel that wrote its partials: the block
+// that takes a tile's last ticket sums them (and returns the counter to zero).
+// The order is that of 256 strided per-thread sums followed by a binary tree
+// over the threads, whatever the number of warps that share the work.
+__device__ __forceinline__ bool last_block(int* ticket, int blocks) {
+  __shared__ int last;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();  // the block's writes, seen through the barrier
+    last = atomicAdd(ticket, 1) == blocks - 1;
+    if (last) {
+      *ticket = 0;
+      __threadfence();
+    }
+  }
+  __syncthreads();
+  return last != 0;
+}
+// one warp; thread slots t = lane + 32 i of the 256, result in lane 0. A
+// slot at or beyond G holds zero, so levels that would only add zeros are
+// skipped.
+__device__ __noinline__ double warp_tree_sum(int G, const double* p) {
+  const int lane = threadIdx.x & 31;
+  double v[8], u[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = lane + 32 * i < G ? __ldcg(p + lane + 32 * i) : 0.0;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) u[i] = 256 + lane + 32 * i < G ? __ldcg(p + 256 + lane + 32 * i) : 0.0;
+  for (int base = 256; base < G; base += 256) {
+    double t[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      t[i] = u[i];
+      const int q = base + 256 + lane + 32 * i;
+      u[i] = q < G ? __ldcg(p + q) : 0.0;
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (base + 32 * i < G) v[i] += t[i];
+  }
+  if (G > 128) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] += v[i + 4];
+  }
+  if (G > 64) {
+    v[0] += v[2];
+    v[1] += v[3];
+  }
+  if (G > 32) v[0] += v[1];
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) v[0] += __shfl_down_sync(0xffffffffu, v[0], off);
+  return v[0];
+}
+// one block of 256 threads, result in thread 0
+__device__ __forceinline__ double block_tree_sum(int G, const double* p, double* sh) {
+  const int t = threadIdx.x;
+  double v = 0.0;
+  int q = t;
+  for (; q + 7 * 256 < G; q += 8 * 256) {
+    double a[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) a[j] = __ldcg(p + q + 256 * j);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v += a[j];
+  }
+  for (; q < G; q += 256) v += __ldcg(p + q);
+  sh[t] = v;
+  __syncthreads();
+  for (int off = 128; off >= 32; off >>= 1) {
+    if (t < off && off < G) sh[t] += sh[t + off];
+    __syncthreads();
+  }
+  v = t < 32 ? sh[t] : 0.0;
+  if (t < 32)
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+  return v;
+}
+
+// Sums over the 32 lanes of M values per lane (M a power of two up to 32),
+// each in the order of a shuffle-down tree (lane l with l + 16, then l + 8,
+// ...): while a lane holds several values, each exchange hands half of them
+// to the partner lane, so every lane adds different values and M sums cost
+// M - 1 + log2(32 / M) additions a lane instead of 5 M. Value
+// lane / (32 / M) ends in v[0].
+template <int M>
+__device__ __forceinline__ void warp_sums(double (&v)[M]) {
+  const int lane = threadIdx.x & 31;
+  int off = 16;
+#pragma unroll
+  for (int h = M / 2; h > 0; h >>= 1) {
+    const bool up = (lane & off) != 0;
+#pragma unroll
+    for (int q = 0; q < h; ++q) {
+      const double send = up ? v[q] : v[q + h], keep = up ? v[q + h] : v[q];
+      v[q] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+    }
+    off >>= 1;
+  }
+  for (; off > 0; off >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], off);
+}
+
+// FP64 multi-dot, out[k] = V[k] . w. The partial sums are those of a fixed
+// grid of G blocks of 256 threads (element i belongs to thread i mod 256 of
+// block (i / 256) mod G), so the result does not depend on the launch:
+// block (x, t) computes the KT vectors of tile t for blocks x, x + gridDim.x,
+// ... of that grid, and a tile's last block to finish sums its
+// partials. mode 1 also adds the sums into aux (second Gram-Schmidt pass).
+//
+// Bound by the FP64 pipe (2 lanes per SM clock; a warp instruction holds its
+// scheduler's unit for 64 clocks): one fma per element is the floor, 2.1 us a
+// vector at 1.08 M rows. The warp trees take 9 FP64 operations per 8 vectors
+// and thread (48 with one tree per vector, against 28 fma). A launch of G
+// blocks, each with its barriers and ticket, cost 25 us before the first fma
+// at 1.08 M rows (three waves of short blocks): here about one wave of blocks
+// shares the grid, and the warps of a block meet once, at its end: 12 us for
+// one vector, about 10 us + 3.1 us a vector for more. With the multi-axpy
+// below, 50 iterations at 1.08 M rows went from 27.6 to 18.2 ms and at
+// 33,792 rows 34 iterations from 3.0 to 1.8 ms.
+constexpr int kMdotPerSm = 3;
+constexpr int kMdotMost = 32;  // fixed-grid blocks per launched block
+
+template <int KT>
+__global__ void __launch_bounds__(kBlock, kMdotPerSm)
+    mdot64_k(int64_t n, int nv, const double* __restrict__ V, int64_t ld, const double* __restrict__ w, int G,
+             double* __restrict__ partial, double* __restrict__ out, double* __restrict__ aux, int mode,
+             int* __restrict__ ticket) {
+  constexpr int M = KT <= 2 ? KT : (KT <= 4 ? 4 : 8);  // sums of a warp's trees
+  constexpr int U = KT <= 2 ? 4 : 2;                   // elements loaded together
+  __shared__ double red[kMdotMost][KT][kBlock / 32];
+  const int64_t stride = int64_t(G) * kBlock;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int k0 = 0; k0 < nv; k0 += kTile) {
-    const int kt = min(kTile, nv - k0);
-    T s[kTile], c[kTile];
+  const int k0 = blockIdx.y * KT, kt = min(KT, nv - k0);
+  const double* __restrict__ Vk = V + int64_t(k0) * ld;
+  int m = 0;
+  for (int b = blockIdx.x; b < G; b += gridDim.x, ++m) {
+    double s[M];
 #pragma unroll
-    for (int k = 0; k < kTile; ++k) s[k] = c[k] = T(0);
-    int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    // two elements per step for more loads in flight
-    for (; i + stride < n; i += 2 * stride) {
-      const T w0 = w[i], w1 = w[i + stride];
-      T a0[kTile], a1[kTile];
+    for (int k = 0; k < M; ++k) s[k] = 0.0;
+    int64_t i = int64_t(b) * kBlock + threadIdx.x;
+    for (; i + (U - 1) * stride < n; i += U * stride) {
+      double x[U], a[U][KT];
 #pragma unroll
-      for (int k = 0; k < kTile; ++k)
-        if (k < kt) {
-          a0[k] = V[int64_t(k0 + k) * ld + i];
-          a1[k] = V[int64_t(k0 + k) * ld + i + stride];
-        }
+      for (int e = 0; e < U; ++e) x[e] = w[i + e * stride];
 #pragma unroll
-      for (int k = 0; k < kTile; ++k)
-        if (k < kt) {
-          acc_prod(a0[k], w0, s[k], c[k]);
-          acc_prod(a1[k], w1, s[k], c[k]);
-        }
+      for (int k = 0; k < KT; ++k)
+        if (k < kt)
+#pragma unroll
+          for (int e = 0; e < U; ++e) a[e][k] = Vk[k * ld + i + e * stride];
+#pragma unroll
+      for (int k = 0; k < KT; ++k)
+        if (k < kt)
+#pragma unroll
+          for (int e = 0; e < U; ++e) s[k] = fma(a[e][k], x[e], s[k]);
     }
-    if (i < n) {
-      const T w0 = w[i];
+    for (; i < n; i += stride) {
+      const double x = w[i];
+      double a[KT];
 #pragma unroll
-      for (int k = 0; k < kTile; ++k)
-        if (k < kt) acc_prod(V[int64_t(k0 + k) * ld + i], w0, s[k], c[k]);
-    }
+      for (int k = 0; k < KT; ++k)
+        if (k < kt) a[k] = Vk[k * ld + i];
 #pragma unroll
-    for (int k = 0; k < kTile; ++k) {
-      if (k < kt) {
-        const double v = warp_sum(s[k], c[k]);
-        if (lane == 0) red[k][warp] = v;
-      }
+      for (int k = 0; k < KT; ++k)
+        if (k < kt) s[k] = fma(a[k], x, s[k]);
     }
-    __syncthreads();
-    if (threadIdx.x < kt) {
-      double v = 0.0;
-      for (int q = 0; q < kBlock / 32; ++q) v += red[threadIdx.x][q];
-      partial[int64_t(k0 + threadIdx.x) * G + blockIdx.x] = v;
+    warp_sums<M>(s);
+    const int k = lane / (32 / M);
+    if (lane % (32 / M) == 0 && k < KT) red[m][k][warp] = s[0];
+  }
+  __syncthreads();
+  for (int q = threadIdx.x; q < m * KT; q += kBlock) {
+    const int k = q % KT, mb = q / KT;
+    if (k < kt) {
+      double v = red[mb][k][0];
+#pragma unroll
+      for (int j = 1; j < kBlock / 32; ++j) v += red[mb][k][j];
+      partial[int64_t(k0 + k) * G + blockIdx.x + mb * gridDim.x] = v;
     }
-    __syncthreads();
+  }
+  if (!last_block(ticket + blockIdx.y, gridDim.x)) return;
+  if (warp < kt) {
+    const int k = k0 + warp;
+    const double v = warp_tree_sum(G, partial + int64_t(k) * G);
+    if (lane == 0) {
+      out[k] = v;
+      if (mode == 1) aux[k] += v;
+    }
   }
 }
 
@@ -271,70 +396,96 @@ __global__ void __launch_bounds__(kBlock)
 // thread with 16-byte loads. Elements in [n, ld) are padding and never
 // enter a result. The multi-dot forms each group of four products with FP32
 // FMAs and adds the group into a compensated (two-float) running sum.
-__global__ void __launch_bounds__(kBlock, 6)
+//
+// Block (b, t) takes tile t of the vectors, and a tile's last block sums its
+// partials: one after the other in a block, the tiles, their barriers and the
+// final sums cost 28 us an iteration at 321 k rows, where a thread has one
+// group or none, against 12 us. The warp trees of a tile's sums run at once, as in warp_sums
+// (the two-sum of a pair does not depend on its order).
+constexpr int kMdot4PerSm = 6;
+__device__ __forceinline__ void pair_add(float& s, float& c, float os, float oc) {
+  c += oc;
+  two_sum_acc(s, c, os);
+}
+__global__ void __launch_bounds__(kBlock, kMdot4PerSm)
     mdot4_k(int64_t n, int nv, const float* __restrict__ V, int64_t ld,
-            const float* __restrict__ w, double* __restrict__ partial) {
+            const float* __restrict__ w, double* __restrict__ partial, double* __restrict__ out,
+            int* __restrict__ ticket) {
   __shared__ double red[kTile][kBlock / 32];
   const int G = gridDim.x;
   const int64_t ng = (n + 3) >> 2, full = n >> 2;  // groups of 4; full groups
   const int64_t stride = int64_t(G) * blockDim.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const float4* w4 = reinterpret_cast<const float4*>(w);
-  for (int k0 = 0; k0 < nv; k0 += kTile) {
-    const int kt = min(kTile, nv - k0);
-    float s[kTile], c[kTile];
+  const int k0 = blockIdx.y * kTile, kt = min(kTile, nv - k0);
+  float s[kTile], c[kTile];
 #pragma unroll
-    for (int k = 0; k < kTile; ++k) s[k] = c[k] = 0.f;
-    for (int64_t g = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; g < ng; g += stride) {
-      float4 wv = w4[g];
-      if (g >= full) {  // the last, partial group
-        const int64_t i0 = 4 * g;
-        if (i0 + 1 >= n) wv.y = 0.f;
-        if (i0 + 2 >= n) wv.z = 0.f;
-        if (i0 + 3 >= n) wv.w = 0.f;
-      }
-#pragma unroll
-      for (int k = 0; k < kTile; ++k)
-        if (k < kt) {
-          float4 a = reinterpret_cast<const float4*>(V + int64_t(k0 + k) * ld)[g];
-          if (g >= full) {
-            const int64_t i0 = 4 * g;
-            if (i0 + 1 >= n) a.y = 0.f;
-            if (i0 + 2 >= n) a.z = 0.f;
-            if (i0 + 3 >= n) a.w = 0.f;
-          }
-          // the group's four products in FP32 (fused), the running sum
-          // compensated: the error is a few ulps of the group's |terms|,
-          // not of the whole length-n sum
-          const float pg = fmaf(a.x, wv.x, fmaf(a.y, wv.y, fmaf(a.z, wv.z, a.w * wv.w)));
-          two_sum_acc(s[k], c[k], pg);
-        }
+  for (int k = 0; k < kTile; ++k) s[k] = c[k] = 0.f;
+  for (int64_t g = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; g < ng; g += stride) {
+    float4 wv = w4[g];
+    if (g >= full) {  // the last, partial group
+      const int64_t i0 = 4 * g;
+      if (i0 + 1 >= n) wv.y = 0.f;
+      if (i0 + 2 >= n) wv.z = 0.f;
+      if (i0 + 3 >= n) wv.w = 0.f;
     }
 #pragma unroll
-    for (int k = 0; k < kTile; ++k) {
+    for (int k = 0; k < kTile; ++k)
       if (k < kt) {
-        const double v = warp_sum(s[k], c[k]);
-        if (lane == 0) red[k][warp] = v;
+        float4 a = reinterpret_cast<const float4*>(V + int64_t(k0 + k) * ld)[g];
+        if (g >= full) {
+          const int64_t i0 = 4 * g;
+          if (i0 + 1 >= n) a.y = 0.f;
+          if (i0 + 2 >= n) a.z = 0.f;
+          if (i0 + 3 >= n) a.w = 0.f;
+        }
+        // the group's four products in FP32 (fused), the running sum
+        // compensated: the error is a few ulps of the group's |terms|,
+        // not of the whole length-n sum
+        const float pg = fmaf(a.x, wv.x, fmaf(a.y, wv.y, fmaf(a.z, wv.z, a.w * wv.w)));
+        two_sum_acc(s[k], c[k], pg);
       }
+  }
+  int off = 16;
+#pragma unroll
+  for (int h = kTile / 2; h > 0; h >>= 1) {
+    const bool up = (lane & off) != 0;
+#pragma unroll
+    for (int q = 0; q < h; ++q) {
+      const float ss = up ? s[q] : s[q + h], sc = up ? c[q] : c[q + h];
+      if (up) {
+        s[q] = s[q + h];
+        c[q] = c[q + h];
+      }
+      pair_add(s[q], c[q], __shfl_xor_sync(0xffffffffu, ss, off), __shfl_xor_sync(0xffffffffu, sc, off));
     }
-    __syncthreads();
-    if (threadIdx.x < kt) {
-      double v = 0.0;
-      for (int q = 0; q < kBlock / 32; ++q) v += red[threadIdx.x][q];
-      partial[int64_t(k0 + threadIdx.x) * G + blockIdx.x] = v;
-    }
-    __syncthreads();
+    off >>= 1;
+  }
+  for (; off > 0; off >>= 1)
+    pair_add(s[0], c[0], __shfl_xor_sync(0xffffffffu, s[0], off), __shfl_xor_sync(0xffffffffu, c[0], off));
+  if ((lane & 3) == 0) red[lane >> 2][warp] = double(s[0]) + double(c[0]);
+  __syncthreads();
+  if (threadIdx.x < kt) {
+    double v = 0.0;
+    for (int q = 0; q < kBlock / 32; ++q) v += red[threadIdx.x][q];
+    partial[int64_t(k0 + threadIdx.x) * G + blockIdx.x] = v;
+  }
+  if (!last_block(ticket + blockIdx.y, G)) return;
+  if (warp < kt) {
+    const double v = warp_tree_sum(G, partial + int64_t(k0 + warp) * G);
+    if (lane == 0) out[k0 + warp] = v;
   }
 }
 
-// w -= V h for groups of four elements; optional per-block partial sums of
-// the updated |w|^2 (elements below n only).
+// w -= V h for groups of four elements, and the norm of the updated w
+// (elements below n only): per-block partial sums of |w|^2, their sum and its
+// root in the last block.
 __global__ void __launch_bounds__(kBlock)
     maxpy4_k(int64_t n, int nv, const float* __restrict__ V, int64_t ld,
              const double* __restrict__ h, float* __restrict__ w,
-             double* __restrict__ nrm_partial) {
+             double* __restrict__ nrm_partial, double* __restrict__ nrm, int* __restrict__ ticket) {
   __shared__ float hs[1024];
-  __shared__ double red[kBlock / 32];
+  __shared__ double red[kBlock / 32], sh[kBlock];
   for (int k = threadIdx.x; k < nv; k += blockDim.x) hs[k] = float(h[k]);
   __syncthreads();
   const int64_t g = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -365,15 +516,12 @@ __global__ void __launch_bounds__(kBlock)
       acc.w = fmaf(-hk, a.w, acc.w);
     }
     reinterpret_cast<float4*>(w)[g] = acc;
-    if (nrm_partial) {
-      const int64_t i0 = 4 * g;
-      acc_prod(acc.x, acc.x, ss, cc);
-      if (i0 + 1 < n) acc_prod(acc.y, acc.y, ss, cc);
-      if (i0 + 2 < n) acc_prod(acc.z, acc.z, ss, cc);
-      if (i0 + 3 < n) acc_prod(acc.w, acc.w, ss, cc);
-    }
+    const int64_t i0 = 4 * g;
+    acc_prod(acc.x, acc.x, ss, cc);
+    if (i0 + 1 < n) acc_prod(acc.y, acc.y, ss, cc);
+    if (i0 + 2 < n) acc_prod(acc.z, acc.z, ss, cc);
+    if (i0 + 3 < n) acc_prod(acc.w, acc.w, ss, cc);
   }
-  if (!nrm_partial) return;
   const double v = warp_sum(ss, cc);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
   __syncthreads();
@@ -382,74 +530,85 @@ __global__ void __launch_bounds__(kBlock)
     for (int q = 0; q < kBlock / 32; ++q) t += red[q];
     nrm_partial[blockIdx.x] = t;
   }
+  if (!last_block(ticket, gridDim.x)) return;
+  const double t = block_tree_sum(gridDim.x, nrm_partial, sh);
+  if (threadIdx.x == 0) nrm[0] = sqrt(t);
 }
 
-// out[k] = sum of partial[k][0..G) (one block per k, fixed tree).
-__global__ void reduce_partials_k(int G, const double* __restrict__ partial,
-                                  double* __restrict__ out, int mode,
-                                  double* __restrict__ aux) {
-  __shared__ double sh[kBlock];
-  const int k = blockIdx.x;
-  double v = 0.0;
-  for (int q = threadIdx.x; q < G; q += blockDim.x)
-    v += partial[int64_t(k) * G + q];
-  sh[threadIdx.x] = v;
-  __syncthreads();
-  for (int off = blockDim.x / 2; off > 0; off >>= 1) {
-    if (threadIdx.x < off) sh[threadIdx.x] += sh[threadIdx.x + off];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    out[k] = sh[0];
-    // mode 1: accumulate into aux[k] (second Gram-Schmidt pass)
-    if (mode == 1) aux[k] += sh[0];
-  }
-}
-
-// w -= sum_k h[k] V[k]  (h on the device, FP64), one element per thread.
-// The coefficients are converted to the vector precision once per block
-// (FP64<->FP32 conversions issue on the narrow FP64 pipe). With
-// nrm_partial != nullptr each block also writes the partial ||w||^2 of its
-// elements to nrm_partial[blockIdx.x].
+// FP64 w -= sum_k h[k] V[k] (h on the device); with nrm, also ||w|| of the
+// result: partial sums per 256 elements (one per thread, warp trees, warps in
+// order), their sum and its root in the last block.
+//
+// EPT elements a thread, 256 apart, so that a thread keeps EPT independent
+// fma chains and loads in flight and the warp trees of EPT partial sums run
+// at once (warp_sums): with one element a thread the trees took 6 FP64
+// operations against one useful product: 23 us with the norm and 8 without at
+// 1.08 M rows and one vector, now 14 and 5. Fewer elements a thread where
+// eight (or four) would leave fewer than three (one) blocks a SM.
 constexpr int kMaxVecs = 1024;
 
-template <typename T>
+template <int EPT>
 __global__ void __launch_bounds__(kBlock)
-    maxpy_k(int64_t n, int nv, const T* __restrict__ V, int64_t ld,
-            const double* __restrict__ h, T* __restrict__ w,
-            double* __restrict__ nrm_partial) {
-  __shared__ T hs[kMaxVecs];
-  __shared__ double red[kBlock / 32];
-  for (int k = threadIdx.x; k < nv; k += blockDim.x) hs[k] = T(h[k]);
+    maxpy64_k(int64_t n, int nv, const double* __restrict__ V, int64_t ld, const double* __restrict__ h,
+              double* __restrict__ w, double* __restrict__ nrm_partial, double* __restrict__ nrm,
+              int* __restrict__ ticket) {
+  __shared__ double hs[kMaxVecs];
+  __shared__ double red[EPT][kBlock / 32], sh[kBlock];
+  for (int k = threadIdx.x; k < nv; k += kBlock) hs[k] = h[k];
   __syncthreads();
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  T ss = T(0), cc = T(0);
-  if (i < n) {
-    T acc = w[i];
+  const int64_t i0 = int64_t(blockIdx.x) * (EPT * kBlock) + threadIdx.x;
+  double acc[EPT];
+  if (i0 + (EPT - 1) * kBlock < n) {
+#pragma unroll
+    for (int e = 0; e < EPT; ++e) acc[e] = w[i0 + e * kBlock];
+    constexpr int U = EPT == 1 ? 8 : (EPT == 4 ? 4 : 2);  // vectors loaded together
     int k = 0;
-    for (; k + 8 <= nv; k += 8) {
-      T a[8];
+    for (; k + U <= nv; k += U) {
+      double a[U][EPT];
 #pragma unroll
-      for (int q = 0; q < 8; ++q) a[q] = V[int64_t(k + q) * ld + i];
+      for (int q = 0; q < U; ++q)
 #pragma unroll
-      for (int q = 0; q < 8; ++q) acc = fma(-hs[k + q], a[q], acc);
+        for (int e = 0; e < EPT; ++e) a[q][e] = V[int64_t(k + q) * ld + i0 + e * kBlock];
+#pragma unroll
+      for (int q = 0; q < U; ++q)
+#pragma unroll
+        for (int e = 0; e < EPT; ++e) acc[e] = fma(-hs[k + q], a[q][e], acc[e]);
     }
-    for (; k < nv; ++k) acc = fma(-hs[k], V[int64_t(k) * ld + i], acc);
-    w[i] = acc;
-    if (nrm_partial) acc_prod(acc, acc, ss, cc);
+    for (; k < nv; ++k)
+#pragma unroll
+      for (int e = 0; e < EPT; ++e) acc[e] = fma(-hs[k], V[int64_t(k) * ld + i0 + e * kBlock], acc[e]);
+#pragma unroll
+    for (int e = 0; e < EPT; ++e) w[i0 + e * kBlock] = acc[e];
+  } else {
+#pragma unroll
+    for (int e = 0; e < EPT; ++e) {
+      const int64_t i = i0 + e * kBlock;
+      acc[e] = 0.0;
+      if (i < n) {
+        acc[e] = w[i];
+        for (int k = 0; k < nv; ++k) acc[e] = fma(-hs[k], V[int64_t(k) * ld + i], acc[e]);
+        w[i] = acc[e];
+      }
+    }
   }
-  if (!nrm_partial) return;
-  const double v = warp_sum(ss, cc);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  if (!nrm) return;
+#pragma unroll
+  for (int e = 0; e < EPT; ++e) acc[e] *= acc[e];
+  warp_sums<EPT>(acc);
+  const int lane = threadIdx.x & 31;
+  if (lane % (32 / EPT) == 0) red[lane / (32 / EPT)][threadIdx.x >> 5] = acc[0];
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0.0;
-    for (int q = 0; q < kBlock / 32; ++q) t += red[q];
-    nrm_partial[blockIdx.x] = t;
+  const int G = int((n + kBlock - 1) / kBlock);
+  if (threadIdx.x < EPT && int(blockIdx.x) * EPT + int(threadIdx.x) < G) {
+    double t = red[threadIdx.x][0];
+#pragma unroll
+    for (int q = 1; q < kBlock / 32; ++q) t += red[threadIdx.x][q];
+    nrm_partial[blockIdx.x * EPT + threadIdx.x] = t;
   }
+  if (!last_block(ticket, gridDim.x)) return;
+  const double t = block_tree_sum(G, nrm_partial, sh);
+  if (threadIdx.x == 0) nrm[0] = sqrt(t);
 }
-
-__global__ void sqrt_scalar_k(double* s) { s[0] = sqrt(s[0]); }
 
 // v32 = float(r / nrm[0]) (start of an inner FP32 cycle).
 __global__ void scale_to_f32_k(int64_t n, const double* __restrict__ r,
@@ -466,25 +625,6 @@ __global__ void jacobi_k(int64_t n, const T* __restrict__ rd,
                          const T* __restrict__ x, T* __restrict__ y) {
   const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i < n) y[i] = x[i] * rd[i];
-}
-
-// v = w / nrm[0] and, when rd is given, z = rd * v (the Jacobi application
-// of the next Arnoldi step) in the same pass.
-template <typename T>
-__global__ void scale_jacobi_k(int64_t n, const T* __restrict__ w,
-                               T* __restrict__ v, const double* __restrict__ nrm,
-                               const T* __restrict__ rd, T* __restrict__ z) {
-  __shared__ T inv;
-  if (threadIdx.x == 0) {
-    const double hn = nrm[0];
-    inv = T(hn != 0.0 ? 1.0 / hn : 0.0);
-  }
-  __syncthreads();
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const T vi = w[i] * inv;
-  v[i] = vi;
-  if (rd) z[i] = vi * rd[i];
 }
 
 constexpr int kGsBatch = 8;
@@ -787,58 +927,117 @@ __global__ void givens_init_k(GivensDev G, double g0) {
 // entry is rel * hist_mul / hist_div; the cycle stops when rel <= tol or
 // hn == 0 (basis j + 1), on a non-finite estimate (basis j + 1) or when the
 // rotation breaks down (basis j).
-__global__ void givens_step_k(GivensDev G, int j, const double* __restrict__ hs,
-                              const double* __restrict__ hnp, double tol, double div,
-                              double hist_mul, double hist_div) {
-  if (threadIdx.x != 0 || G.ctl[kCtlDone]) return;
-  const int m = G.m;
+struct GivensCol {
+  GivensDev G;
+  int j;
+  const double *hs, *hn;
+  double tol, div, hist_mul, hist_div;
+};
+
+// By one warp. The rotations are a serial chain a <- c_k h_{k+1} - s_k a; the
+// products with h and the entries of the column are formed by 32 lanes at a
+// time, so a rotation costs one multiply and one add of latency (0.14 us)
+// instead of a load of the previous store and six operations (0.5 us).
+__device__ void givens_step(const GivensCol& c) {
+  const GivensDev& G = c.G;
+  const int lane = threadIdx.x & 31;
+  if (G.ctl[kCtlDone]) return;
+  const int m = G.m, j = c.j;
   double* H = G.H;
-  const double hn = hnp[0];
-  for (int k = 0; k <= j; ++k) H[size_t(k) * m + j] = hs[k];
-  H[size_t(j + 1) * m + j] = hn;
-  for (int k = 0; k < j; ++k) {
-    const double a = H[size_t(k) * m + j], bb = H[size_t(k + 1) * m + j];
-    H[size_t(k) * m + j] = __dadd_rn(__dmul_rn(G.cs[k], a), __dmul_rn(G.sn[k], bb));
-    H[size_t(k + 1) * m + j] = __dadd_rn(__dmul_rn(-G.sn[k], a), __dmul_rn(G.cs[k], bb));
+  const double hn = c.hn[0];
+  double a = c.hs[0];
+  for (int k0 = 0; k0 < j; k0 += 32) {
+    const int k = k0 + lane;
+    const bool on = k < j;
+    const double cs = on ? G.cs[k] : 0.0, sn = on ? G.sn[k] : 0.0, h = on ? c.hs[k + 1] : 0.0;
+    const double p = __dmul_rn(sn, h), q = __dmul_rn(cs, h);
+    double ak = 0.0;
+    const int cnt = min(32, j - k0);
+    for (int l = 0; l < cnt; ++l) {
+      const double snl = __shfl_sync(0xffffffffu, sn, l), ql = __shfl_sync(0xffffffffu, q, l);
+      if (lane == l) ak = a;
+      a = __dadd_rn(__dmul_rn(-snl, a), ql);
+    }
+    if (on) H[size_t(k) * m + j] = __dadd_rn(__dmul_rn(cs, ak), p);
   }
-  const double a = H[size_t(j) * m + j], bb = H[size_t(j + 1) * m + j];
+  if (lane != 0) return;
+  const double bb = hn;
   const double den = __dsqrt_rn(__dadd_rn(__dmul_rn(a, a), __dmul_rn(bb, bb)));
+  H[size_t(j) * m + j] = a;
+  H[size_t(j + 1) * m + j] = bb;
   if (!(den > 0.0) || !isfinite(den)) {
     G.ctl[kCtlStatus] = isfinite(den) ? NW_BREAKDOWN : NW_NAN_DETECTED;
     G.ctl[kCtlBasis] = j;
     G.ctl[kCtlDone] = 1;
     return;
   }
-  G.cs[j] = __ddiv_rn(a, den);
-  G.sn[j] = __ddiv_rn(bb, den);
+  const double cj = __ddiv_rn(a, den), sj = __ddiv_rn(bb, den);
+  G.cs[j] = cj;
+  G.sn[j] = sj;
   H[size_t(j) * m + j] = den;
   H[size_t(j + 1) * m + j] = 0.0;
-  G.g[j + 1] = __dmul_rn(-G.sn[j], G.g[j]);
-  G.g[j] = __dmul_rn(G.cs[j], G.g[j]);
+  const double gj = G.g[j], gn = __dmul_rn(-sj, gj);
+  G.g[j + 1] = gn;
+  G.g[j] = __dmul_rn(cj, gj);
   G.ctl[kCtlIts] = j + 1;
-  const double rel = __ddiv_rn(fabs(G.g[j + 1]), div);
-  G.hist[j] = __ddiv_rn(__dmul_rn(rel, hist_mul), hist_div);
+  const double rel = __ddiv_rn(fabs(gn), c.div);
+  G.hist[j] = __ddiv_rn(__dmul_rn(rel, c.hist_mul), c.hist_div);
   if (!isfinite(rel)) {
     G.ctl[kCtlStatus] = NW_NAN_DETECTED;
     G.ctl[kCtlBasis] = j + 1;
     G.ctl[kCtlDone] = 1;
-  } else if (rel <= tol || hn == 0.0) {
+  } else if (rel <= c.tol || hn == 0.0) {
     G.ctl[kCtlBasis] = j + 1;
     G.ctl[kCtlDone] = 1;
   }
 }
 
+// v = w / nrm[0] and, when rd is given, z = rd * v (the Jacobi application
+// of the next Arnoldi step) in the same pass. GIVENS: block 0 instead applies
+// the Givens rotations to the new Hessenberg column, beside the scaling.
+template <typename T, bool GIVENS>
+__global__ void __launch_bounds__(kBlock)
+    scale_jacobi_k(int64_t n, const T* __restrict__ w, T* __restrict__ v, const double* __restrict__ nrm,
+                   const T* __restrict__ rd, T* __restrict__ z, GivensCol gc) {
+  if (GIVENS && blockIdx.x == 0) {
+    if (threadIdx.x < 32) givens_step(gc);
+    return;
+  }
+  __shared__ T inv;
+  if (threadIdx.x == 0) {
+    const double hn = nrm[0];
+    inv = T(hn != 0.0 ? 1.0 / hn : 0.0);
+  }
+  __syncthreads();
+  const int64_t i = int64_t(blockIdx.x - (GIVENS ? 1 : 0)) * kBlock + threadIdx.x;
+  if (i >= n) return;
+  const T vi = w[i] * inv;
+  v[i] = vi;
+  if (rd) z[i] = vi * rd[i];
+}
+
 // Back substitution H(0:kk, 0:kk) y = g(0:kk), y scaled by yscale, into y.
+// Row i subtracts H(i, l) y(l) in ascending l, so its chain of subtractions
+// starts when y(i + 1) is known and is serial; the products are formed by the
+// 32 lanes (154 us for 50 columns with one thread's loads and multiplies in
+// the chain).
 __global__ void givens_solve_k(GivensDev G, int kk, double yscale, double* __restrict__ y) {
-  if (threadIdx.x != 0) return;
-  const int m = G.m;
+  __shared__ double ys[kMaxVecs];
+  const int m = G.m, lane = threadIdx.x;
   for (int i = kk - 1; i >= 0; --i) {
     double sum = G.g[i];
-    for (int l = i + 1; l < kk; ++l) sum = __dsub_rn(sum, __dmul_rn(G.H[size_t(i) * m + l], y[l]));
-    y[i] = __ddiv_rn(sum, G.H[size_t(i) * m + i]);
+    const double d = G.H[size_t(i) * m + i];
+    for (int l0 = i + 1; l0 < kk; l0 += 32) {
+      const int l = l0 + lane, cnt = min(32, kk - l0);
+      const double p = l < kk ? __dmul_rn(G.H[size_t(i) * m + l], ys[l]) : 0.0;
+#pragma unroll 4
+      for (int q = 0; q < cnt; ++q) sum = __dsub_rn(sum, __shfl_sync(0xffffffffu, p, q));
+    }
+    const double v = __ddiv_rn(sum, d);
+    if (lane == 0) ys[i] = v;
+    __syncwarp();
   }
-  if (yscale != 1.0)
-    for (int i = 0; i < kk; ++i) y[i] = __dmul_rn(y[i], yscale);
+  for (int i = lane; i < kk; i += 32) y[i] = yscale != 1.0 ? __dmul_rn(ys[i], yscale) : ys[i];
 }
 
 }  // namespace
@@ -858,10 +1057,7 @@ KrylovSolver::Cycle KrylovSolver::run_cycle(int m, int max_steps, double g0, dou
   givens_init_k<<<1, 32, 0, s>>>(G, g0);
   int launched = 0, pending = -1, slot = 0;
   bool stop = false;
-  auto step = [&](int j) {
-    arnoldi(j);
-    givens_step_k<<<1, 32, 0, s>>>(G, j, hs, hn, tol, div, hist_mul, hist_div);
-  };
+  auto step = [&](int j) { arnoldi(j, GivensCol{G, j, hs, hn, tol, div, hist_mul, hist_div}); };
   for (int j = 0; j < m && launched < max_steps && !stop; ++j) {
     // the first step of a cycle runs as plain launches: any one-time set-up
     // (buffer growth) happens there, outside a capture. A stream that cannot
@@ -954,12 +1150,12 @@ void KrylovSolver::setup(const DevCsr& A, int m, cudaStream_t s) {
   NW_CUDA(cudaGetDevice(&dev));
   int sms = 0;
   NW_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  sms_ = sms;
   red_blocks_ = int(std::max<int64_t>(1, std::min<int64_t>(8 * sms, (n + 2 * kBlock - 1) / (2 * kBlock))));
-  // the FP32 multi-dot holds 16 accumulators per thread: size its grid to
-  // the blocks that are resident at once (one wave of its grid-stride loop)
-  int occ = 0;
-  NW_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, mdot4_k, kBlock, 0));
-  mdot4_blocks_ = std::max(1, std::min(red_blocks_, std::max(1, occ) * sms));
+  // the FP32 multi-dot holds 16 accumulators per thread: its grid is the
+  // blocks that are resident at once (one wave of its grid-stride loop). Both
+  // grids also fix the order of the sums.
+  mdot4_blocks_ = std::min(red_blocks_, kMdot4PerSm * sms);
   rdiag_.resize(n);
   V_.resize(size_t(m_ + 1) * n);
   Z_.release();
@@ -974,6 +1170,8 @@ void KrylovSolver::setup(const DevCsr& A, int m, cudaStream_t s) {
     if (!e) NW_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   gst_.resize(size_t(m_ + 1) * m_ + 4 * size_t(m_) + 1);
   gctl_.resize(4);
+  ticket_.resize(size_t(m_) / kTile + 2);
+  NW_CUDA(cudaMemsetAsync(ticket_.p, 0, ticket_.n * sizeof(int), s));
   // sliced-ELL layout from the host CSR
   sell_slices_ = 0;
   if (A.row_ptr_host && A.col_idx_host && n > 0) {
@@ -1095,10 +1293,45 @@ void KrylovSolver::spmv32(const float* x, float* y, cudaStream_t s) const {
   }
 }
 
+// out[k] = V[k] . w, k < nv; with acc also acc[k] += out[k]
+void KrylovSolver::mdot64(int nv, const double* V, int64_t ld, const double* w, double* out, double* acc,
+                          cudaStream_t s) {
+  if (nv < 1) return;
+  // tiles of equal width: 25 vectors are 7 + 7 + 7 + 4
+  const int tiles = (nv + kTile - 1) / kTile, kt = (nv + tiles - 1) / tiles, wave = kMdotPerSm * sms_;
+  // fixed-grid blocks per launched block: about one wave of blocks in all
+  const int per = std::min(kMdotMost, std::max(1, (red_blocks_ * tiles + wave / 2) / wave));
+  const dim3 grid(unsigned((red_blocks_ + per - 1) / per), unsigned((nv + kt - 1) / kt));
+  auto launch = [&](auto kernel) {
+    kernel<<<grid, kBlock, 0, s>>>(A_.n, nv, V, ld, w, red_blocks_, partial_.p, out, acc, acc ? 1 : 0, ticket_.p);
+  };
+  switch (kt) {
+    case 1: launch(mdot64_k<1>); break;
+    case 2: launch(mdot64_k<2>); break;
+    case 3: launch(mdot64_k<3>); break;
+    case 4: launch(mdot64_k<4>); break;
+    case 5: launch(mdot64_k<5>); break;
+    case 6: launch(mdot64_k<6>); break;
+    case 7: launch(mdot64_k<7>); break;
+    default: launch(mdot64_k<8>); break;
+  }
+}
+
+// w -= sum_k h[k] V[k]; with nrm also nrm[0] = ||w||
+void KrylovSolver::maxpy64(int nv, const double* V, int64_t ld, const double* h, double* w, double* nrm,
+                           cudaStream_t s) {
+  const int64_t n = A_.n;
+  const unsigned g = grid1(n);
+  if (g >= unsigned(8 * 3 * sms_))
+    maxpy64_k<8><<<(g + 7) / 8, kBlock, 0, s>>>(n, nv, V, ld, h, w, partial_.p, nrm, ticket_.p);
+  else if (g >= unsigned(4 * sms_))
+    maxpy64_k<4><<<(g + 3) / 4, kBlock, 0, s>>>(n, nv, V, ld, h, w, partial_.p, nrm, ticket_.p);
+  else
+    maxpy64_k<1><<<g, kBlock, 0, s>>>(n, nv, V, ld, h, w, partial_.p, nrm, ticket_.p);
+}
+
 double KrylovSolver::dot(const double* a, const double* b, cudaStream_t s) {
-  mdot_k<double><<<red_blocks_, kBlock, 0, s>>>(A_.n, 1, a, 0, b, partial_.p);
-  reduce_partials_k<<<1, kBlock, 0, s>>>(red_blocks_, partial_.p, scal_.p, 0,
-                                         nullptr);
+  mdot64(1, a, 0, b, scal_.p, nullptr, s);
   NW_CUDA(cudaMemcpyAsync(h_pinned_, scal_.p, sizeof(double),
                           cudaMemcpyDeviceToHost, s));
   NW_CUDA(cudaStreamSynchronize(s));
@@ -1535,25 +1768,21 @@ SolveResult KrylovSolver::gmres(const nw_solver_cfg& cfg, double tol,
   while (!done && its < cfg.max_iterations) {
     // V0 = r / beta (and z0 = D^-1 V0)
     NW_CUDA(cudaMemcpyAsync(h2, &beta, sizeof(double), cudaMemcpyHostToDevice, s));
-    scale_jacobi_k<double><<<grid1(n), kBlock, 0, s>>>(
-        n, r_.p, V, h2, fuse_jacobi ? rdiag_.p : nullptr, flexible ? Z_.p : z_.p);
-    auto arnoldi = [&](int j) {
+    scale_jacobi_k<double, false><<<grid1(n), kBlock, 0, s>>>(
+        n, r_.p, V, h2, fuse_jacobi ? rdiag_.p : nullptr, flexible ? Z_.p : z_.p, GivensCol{});
+    auto arnoldi = [&](int j, const GivensCol& gc) {
       double* vj = V + size_t(j) * n;
       double* zj = flexible ? Z_.p + size_t(j) * n : z_.p;
       if (!fuse_jacobi) apply_precond(pc, vj, zj, s);
       spmv(zj, w_.p, s);
       // two classical Gram-Schmidt passes, coefficients kept on the device
-      mdot_k<double><<<red_blocks_, kBlock, 0, s>>>(n, j + 1, V, n, w_.p, partial_.p);
-      reduce_partials_k<<<j + 1, kBlock, 0, s>>>(red_blocks_, partial_.p, hs, 0, nullptr);
-      maxpy_k<double><<<grid1(n), kBlock, 0, s>>>(n, j + 1, V, n, hs, w_.p, nullptr);
-      mdot_k<double><<<red_blocks_, kBlock, 0, s>>>(n, j + 1, V, n, w_.p, partial_.p);
-      reduce_partials_k<<<j + 1, kBlock, 0, s>>>(red_blocks_, partial_.p, h2 + 1, 1, hs);
-      maxpy_k<double><<<grid1(n), kBlock, 0, s>>>(n, j + 1, V, n, h2 + 1, w_.p, partial_.p);
-      reduce_partials_k<<<1, kBlock, 0, s>>>(int(grid1(n)), partial_.p, h2, 0, nullptr);
-      sqrt_scalar_k<<<1, 1, 0, s>>>(h2);
+      mdot64(j + 1, V, n, w_.p, hs, nullptr, s);
+      maxpy64(j + 1, V, n, hs, w_.p, nullptr, s);
+      mdot64(j + 1, V, n, w_.p, h2 + 1, hs, s);
+      maxpy64(j + 1, V, n, h2 + 1, w_.p, h2, s);
       double* znext = (j + 1 < m) ? (flexible ? Z_.p + size_t(j + 1) * n : z_.p) : nullptr;
-      scale_jacobi_k<double><<<grid1(n), kBlock, 0, s>>>(
-          n, w_.p, V + size_t(j + 1) * n, h2, (fuse_jacobi && znext) ? rdiag_.p : nullptr, znext);
+      scale_jacobi_k<double, true><<<grid1(n) + 1, kBlock, 0, s>>>(
+          n, w_.p, V + size_t(j + 1) * n, h2, (fuse_jacobi && znext) ? rdiag_.p : nullptr, znext, gc);
     };
     const Cycle c = run_cycle(m, cfg.max_iterations - its, beta, tol, bnorm, 1.0, 1.0, arnoldi, hs, h2, s);
     its += c.iterations;
@@ -1652,7 +1881,7 @@ SolveResult KrylovSolver::sstep_gmres(const nw_solver_cfg& cfg, double tol, cons
   };
   while (!done && its < cfg.max_iterations) {
     upload(h2, &beta, 1);
-    scale_jacobi_k<double><<<grid1(n), kBlock, 0, s>>>(n, r_.p, V, h2, nullptr, nullptr);
+    scale_jacobi_k<double, false><<<grid1(n), kBlock, 0, s>>>(n, r_.p, V, h2, nullptr, nullptr, GivensCol{});
     std::fill(H.begin(), H.end(), 0.0);
     std::fill(Hr.begin(), Hr.end(), 0.0);
     std::fill(g.begin(), g.end(), 0.0);
@@ -1667,18 +1896,15 @@ SolveResult KrylovSolver::sstep_gmres(const nw_solver_cfg& cfg, double tol, cons
         double* w = W + size_t(k) * n;
         apply_precond(pc, V + size_t(j0 + k) * n, z_.p, s);
         spmv(z_.p, w, s);
-        scale_jacobi_k<double><<<grid1(n), kBlock, 0, s>>>(n, w, w, Sd, nullptr, nullptr);
+        scale_jacobi_k<double, false><<<grid1(n), kBlock, 0, s>>>(n, w, w, Sd, nullptr, nullptr, GivensCol{});
       }
       // two block classical Gram-Schmidt passes against V(:, 0:j0+1)
       std::fill(Ch.begin(), Ch.end(), 0.0);
       for (int pass = 0; pass < 2; ++pass) {
-        for (int k = 0; k < sb; ++k) {
-          mdot_k<double><<<red_blocks_, kBlock, 0, s>>>(n, j0 + 1, V, n, W + size_t(k) * n, partial_.p);
-          reduce_partials_k<<<j0 + 1, kBlock, 0, s>>>(red_blocks_, partial_.p, Cd + size_t(k) * ldc, 0, nullptr);
-        }
         for (int k = 0; k < sb; ++k)
-          maxpy_k<double><<<grid1(n), kBlock, 0, s>>>(n, j0 + 1, V, n, Cd + size_t(k) * ldc,
-                                                      W + size_t(k) * n, nullptr);
+          mdot64(j0 + 1, V, n, W + size_t(k) * n, Cd + size_t(k) * ldc, nullptr, s);
+        for (int k = 0; k < sb; ++k)
+          maxpy64(j0 + 1, V, n, Cd + size_t(k) * ldc, W + size_t(k) * n, nullptr, s);
         download(Cp.data(), Cd, size_t(ldc) * sb);
         for (int k = 0; k < sb; ++k)
           for (int i = 0; i <= j0; ++i) Ch[size_t(k) * ldc + i] += Cp[size_t(k) * ldc + i];
@@ -1688,10 +1914,7 @@ SolveResult KrylovSolver::sstep_gmres(const nw_solver_cfg& cfg, double tol, cons
       for (int k = 0; k < sb; ++k) Rt[size_t(k) * sb + k] = 1.0;  // Rt[i][k] at k sb + i
       bool broke = false;
       for (int pass = 0; pass < 2 && !broke; ++pass) {
-        for (int k = 0; k < sb; ++k) {
-          mdot_k<double><<<red_blocks_, kBlock, 0, s>>>(n, sb, W, n, W + size_t(k) * n, partial_.p);
-          reduce_partials_k<<<sb, kBlock, 0, s>>>(red_blocks_, partial_.p, Gd + size_t(k) * sstep, 0, nullptr);
-        }
+        for (int k = 0; k < sb; ++k) mdot64(sb, W, n, W + size_t(k) * n, Gd + size_t(k) * sstep, nullptr, s);
         download(Gh.data(), Gd, size_t(sstep) * sb);
         std::fill(Rp.begin(), Rp.end(), 0.0);
         for (int k = 0; k < sb && !broke; ++k) {
@@ -1713,10 +1936,10 @@ SolveResult KrylovSolver::sstep_gmres(const nw_solver_cfg& cfg, double tol, cons
           double* w = W + size_t(k) * n;
           if (k > 0) {
             upload(Rd, &Rp[size_t(k) * sb], size_t(k));
-            maxpy_k<double><<<grid1(n), kBlock, 0, s>>>(n, k, W, n, Rd, w, nullptr);
+            maxpy64(k, W, n, Rd, w, nullptr, s);
           }
           upload(Sd, &Rp[size_t(k) * sb + k], 1);
-          scale_jacobi_k<double><<<grid1(n), kBlock, 0, s>>>(n, w, w, Sd, nullptr, nullptr);
+          scale_jacobi_k<double, false><<<grid1(n), kBlock, 0, s>>>(n, w, w, Sd, nullptr, nullptr, GivensCol{});
         }
         // Rt = Rp Rt (both upper triangular)
         for (int k = 0; k < sb; ++k)
@@ -2100,7 +2323,7 @@ SolveResult KrylovSolver::mixed(const nw_solver_cfg& cfg, double tol,
     scale_to_f32_k<<<grid1(n), kBlock, 0, s>>>(n, r_.p, V, h2);
     if (fuse_jacobi) jacobi_k<float><<<grid1(n), kBlock, 0, s>>>(n, rdiag32_.p, V, z32_.p);
     // inner system solved for r / ||r|| (g0 = 1)
-    auto arnoldi = [&](int j) {
+    auto arnoldi = [&](int j, const GivensCol& gc) {
       float* vj = V + size_t(j) * ld;
       float* zj = flexible ? Z32_.p + size_t(j) * ld : z32_.p;
       if (!fuse_jacobi) precond32(pc, vj, zj, s);
@@ -2110,13 +2333,10 @@ SolveResult KrylovSolver::mixed(const nw_solver_cfg& cfg, double tol,
       // cycle and the FP64 outer loop recomputes the true residual, so the
       // second pass of the FP64 method is not needed here (same iteration
       // counts on the Poisson systems measured)
-      mdot4_k<<<mdot4_blocks_, kBlock, 0, s>>>(n, j + 1, V, ld, w32_.p, partial_.p);
-      reduce_partials_k<<<j + 1, kBlock, 0, s>>>(mdot4_blocks_, partial_.p, hs, 0, nullptr);
-      maxpy4_k<<<g4, kBlock, 0, s>>>(n, j + 1, V, ld, hs, w32_.p, partial_.p);
-      reduce_partials_k<<<1, kBlock, 0, s>>>(int(g4), partial_.p, h2, 0, nullptr);
-      sqrt_scalar_k<<<1, 1, 0, s>>>(h2);
-      scale_jacobi_k<float><<<grid1(n), kBlock, 0, s>>>(n, w32_.p, V + size_t(j + 1) * ld, h2,
-                                                        fuse_jacobi ? rdiag32_.p : nullptr, z32_.p);
+      mdot4_k<<<dim3(mdot4_blocks_, j / kTile + 1), kBlock, 0, s>>>(n, j + 1, V, ld, w32_.p, partial_.p, hs, ticket_.p);
+      maxpy4_k<<<g4, kBlock, 0, s>>>(n, j + 1, V, ld, hs, w32_.p, partial_.p, h2, ticket_.p);
+      scale_jacobi_k<float, true><<<grid1(n) + 1, kBlock, 0, s>>>(n, w32_.p, V + size_t(j + 1) * ld, h2,
+                                                                  fuse_jacobi ? rdiag32_.p : nullptr, z32_.p, gc);
     };
     const Cycle c = run_cycle(m, cfg.max_iterations - its, 1.0, itol, 1.0, rnorm, bnorm, arnoldi, hs, h2, s,
                               true);

@@ -138,9 +138,10 @@ class KrylovSolver {
     nw_status status = NW_OK;
     std::vector<double> hist;
   };
-  // One restart cycle's Arnoldi steps (arnoldi(j) launches iteration j's
-  // kernels, ending with the new column in hs[0..j] and its norm at h2[0])
-  // with the Givens update on the device and the host one chunk behind.
+  // One restart cycle's Arnoldi steps (arnoldi(j, column) launches iteration
+  // j's kernels: the new column in hs[0..j], its norm at hn[0], then the
+  // column's Givens update beside the scaling of the new vector), with the
+  // host one chunk behind.
   // With `graph`, the steps after the first of the cycle are captured from
   // the same launches into a CUDA graph each, which updates iter_exec_ in
   // place and is launched as one unit (the kernels then follow each other
@@ -201,6 +202,10 @@ class KrylovSolver {
   DeviceArray<float> vals32_, rdiag32_, V32_, w32_, z32_, r32_;
   int64_t ld32_ = 0;  // leading dimension of the FP32 basis (n rounded up to 32)
   bool f32_valid_ = false;
+  void mdot64(int nv, const double* V, int64_t ld, const double* w, double* out, double* acc, cudaStream_t s);
+  void maxpy64(int nv, const double* V, int64_t ld, const double* h, double* w, double* nrm, cudaStream_t s);
+  DeviceArray<int> ticket_;   // finished blocks per tile of a reduction (zero between launches)
+  int sms_ = 1;
   int red_blocks_ = 0;
   int mdot4_blocks_ = 0;  // grid of the FP32 multi-dot (one resident wave)
 };
