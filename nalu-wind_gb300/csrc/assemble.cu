@@ -29,6 +29,7 @@
 // template parameters.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <type_traits>
 
@@ -43,6 +44,7 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kRow1Threads = 128;  // node rows per block, 1-dof row phase
 constexpr int kMaxRowSmem = 96 * 1024;  // staging capacity limit per block
+constexpr int kSmSmem = 228 * 1024;     // shared memory of a SM
 
 // 1/x from the MUFU approximation (rcp.approx.ftz.f64) refined by a cubic
 // step r(1 + e + e^2) and a Newton step r(1 + e), e = 1 - x r. Zero,
@@ -320,13 +322,30 @@ __device__ __forceinline__ dd van_leer_dd(dd dqm, dd dqp, dd eps) {
 //   LL = cLL I - N/relax,  LR = cLR I + N,  RL = cRL I + N,
 //   RR = cRR I - N/relax,  N_ij = -viscIp A_i A_j / (A.dx)
 // because the advective and diffusive factors do not depend on the
-// component; the rhs is (-tf, +tf). In float-float arithmetic negation is
-// exact and addition and multiplication are odd, so cLL = -cRL / relax and
-// cRR = -cLR / relax hold bit for bit: the row phase derives the diagonal
-// constants and the edge phase stores 11 SoA arrays of float pairs per
-// edge: cLR, cRL, N00, N01, N02, N11, N12, N22, tf0, tf1, tf2.
+// component; the rhs is (-tf, +tf), and cLL = -cRL / relax, cRR = -cLR /
+// relax. So an off-diagonal CSR entry is N_ij or N_qq + c of one edge, and a
+// diagonal block is -(the sum over the row's edges of the opposite block) /
+// relax. The edge phase writes the nine distinct entries as the FP64 numbers
+// that go into the matrix, widened once here instead of once per row and
+// component, and the three fluxes as float pairs: a 96-byte record
+//   D_LR0 D_RL0 tf0 N01 | D_LR1 D_RL1 tf1 N12 | D_LR2 D_RL2 tf2 N02
+// (D_LRq = N_qq + c_LR), one 32-byte sector per component: what the row
+// thread of that component needs but for one entry of N.
+//
+// Both FP32 issue and the FP64 pipe work here: sums and differences of FP64
+// inputs are one FP64 operation each (25 an edge, 64 clocks of a scheduler's
+// unit), exact to 53 bits, and replace the pair additions (11 operations) and
+// second splits; products stay in float pairs. With g = grad u_L + grad u_R
+// and the upwind side's gradient (the only one the default options need) an
+// edge takes 1,900 instructions; the form that split every operand and added
+// in pairs took 2,200. At 128 x 128 x 64 this kernel went from 309 to 267 us
+// (59 % issue, FP64 pipe busy half the time) and the row kernel below from
+// 228 to 172; on 734,831 edges of randomly numbered tets, where eleven arrays
+// meant eleven sectors an edge and side, from 100 to 76 and from 232 to 59.
+// The whole assembly: 542 -> 449 us and 331 -> 139 us, with smaller errors
+// against 64 bits in values and rhs.
 struct MomentumDD {
-  dd alpha, alpha_upw, om_alpha, om_alpha_upw, upw, divu_fac, irelax, eps;
+  dd alpha, alpha_upw, om_alpha, om_alpha_upw, upw, divu_fac, eps;
 };
 
 struct MomentumIn {
@@ -341,140 +360,136 @@ struct MomentumIn {
   const double* __restrict__ pec;
 };
 
+// 32 bytes at once (p 32-byte aligned)
+__device__ __forceinline__ void st32(double* p, double a, double b, double c, double d) {
+  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(a), "d"(b), "d"(c), "d"(d) : "memory");
+}
+__device__ __forceinline__ double pair_bits(dd a) {
+  return __hiloint2double(__float_as_int(a.lo), __float_as_int(a.hi));
+}
+
 // DEF: the reference's default advection options alpha = 0, alpha_upw = 1,
-// upw_factor = 1 (SolutionOptions, src/SolutionOptions.C:31-80). The general
-// formulas then multiply by exactly one and add exact zeros, which in
-// float-float arithmetic return their operand unchanged, so the
-// specialisation drops those operations and gives the same bits.
+// upw_factor = 1 (SolutionOptions, src/SolutionOptions.C:31-80): only the
+// upwind side's extrapolation enters, as its difference from the edge mean.
 template <bool LIMITER, bool DIVU, bool DEF>
-__device__ __forceinline__ void momentum_edge(int64_t e, int64_t E, const MomentumIn& in,
-                                              const MomentumDD& c, dd* __restrict__ b) {
-  const int2* __restrict__ edges = in.edges;
+__device__ __forceinline__ void momentum_edge(int64_t e, const MomentumIn& in, const MomentumDD& c,
+                                              double* __restrict__ rec) {
   const double* __restrict__ coords = in.coords;
   const double* __restrict__ vel = in.vel;
   const double* __restrict__ dudx = in.dudx;
-  const double* __restrict__ viscosity = in.viscosity;
-  const double* __restrict__ mask = in.mask;
-  const double* __restrict__ area = in.area;
-  const double* __restrict__ mdotA = in.mdot;
-  const double* __restrict__ pecA = in.pec;
-  const int2 lr = edges[e];
+  const int2 lr = in.edges[e];
   // 32-bit node offsets (9 N < 2^32 is checked when the system is
   // finalized): fewer registers than 64-bit ones
   const uint32_t L = uint32_t(lr.x), R = uint32_t(lr.y);
-  // coordinate and velocity differences are formed in FP64 and split once:
-  // splitting each operand to a float pair first would keep only 48 bits of
-  // each, and the difference of nearby values would lose the rest
-  dd av[3], dx[3], uL[3], uR[3], du[3];
+  dd av[3], hdx[3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
-    av[d] = ldd(area + 3 * e + d);
-    dx[d] = dd_from_double(coords[3 * R + d] - coords[3 * L + d]);
-    uL[d] = ldd(vel + 3 * L + d);
-    uR[d] = ldd(vel + 3 * R + d);
-    du[d] = dd_from_double(vel[3 * R + d] - vel[3 * L + d]);
+    av[d] = dd_from_double_z(in.area[3 * e + d]);
+    hdx[d] = scale2(dd_from_double_z(coords[3 * R + d] - coords[3 * L + d]), 0.5f);
   }
-  const dd mdot = ldd(mdotA + e);
-  const dd viscIp = scale2(ldd(viscosity + L) + ldd(viscosity + R), 0.5f);
+  // the advective flux mdot u carries the largest terms of the rhs: its two
+  // factors are split to the nearest pair (errors against 64 bits 1.9e-14 ->
+  // 1.3e-14 of the rhs norm at 128 x 128 x 64)
+  const dd mdot = dd_from_double_near(in.mdot[e]), pec = ldd(in.pec + e);
+  const bool up = dd_gt0(mdot);
   const dd asq = dd_dot3(av[0], av[0], av[1], av[1], av[2], av[2]);
-  const dd axdx = dd_dot3(av[0], dx[0], av[1], dx[1], av[2], dx[2]);
-  const dd inv_axdx = dd_rcp(axdx);
-  dd hdx[3];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) hdx[d] = scale2(dx[d], 0.5f);
-  // duidxj with the over-relaxed non-orthogonal correction (gj holds the
-  // sum, not the mean, of the two nodal gradients); duL / duR are the
-  // extrapolation increments 0.5 dx . grad u of each side, and their sum is
-  // the correction's 0.5 dx . (grad u_L + grad u_R)
-  dd duidxj[3][3], duL[3], duR[3];
+  const dd hinv = dd_rcp(dd_dot3(av[0], hdx[0], av[1], hdx[1], av[2], hdx[2]));  // 2 / (A.dx)
+  const dd inv_axdx = scale2(hinv, 0.5f);
+  const dd mp = mdot * pec;
+  // g: the sum (not the mean) of the two nodal gradients; corr: the factor of
+  // the over-relaxed non-orthogonal correction, duidxj = g / 2 + corr A; adv:
+  // the advective flux
+  dd g[3][3], corr[3], adv[3];
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    dd gl[3], gr[3], gj[3];
+    const double uL = vel[3 * L + i], uR = vel[3 * R + i];
+    double gl[3], gr[3], gs[3];
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
-      gl[j] = ldd(dudx + 9 * L + 3 * i + j);
-      gr[j] = ldd(dudx + 9 * R + 3 * i + j);
-      gj[j] = gr[j] + gl[j];
+      gl[j] = dudx[9 * L + 3 * i + j];
+      gr[j] = dudx[9 * R + 3 * i + j];
+      gs[j] = gl[j] + gr[j];
     }
-    duL[i] = dd_dot3(hdx[0], gl[0], hdx[1], gl[1], hdx[2], gl[2]);
-    duR[i] = dd_dot3(hdx[0], gr[0], hdx[1], gr[1], hdx[2], gr[2]);
-    const dd gjuidx = duL[i] + duR[i];
-    const dd corr = (du[i] - gjuidx) * inv_axdx;
-#pragma unroll
-    for (int j = 0; j < 3; ++j) duidxj[i][j] = corr * av[j] + scale2(gj[j], 0.5f);
-  }
-  dd limitL[3], limitR[3];
-  if (LIMITER) {
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      limitL[d] = van_leer_dd(scale2(duL[d], 4.0f) - du[d], du[d], c.eps);
-      limitR[d] = van_leer_dd(scale2(duR[d], 4.0f) - du[d], du[d], c.eps);
-    }
-  }
-  const dd pecfac = ldd(pecA + e);
-  const dd om_pecfac = dd{1.0f, 0.0f} - pecfac;
-  const dd maskNode = dd_min(ldd(mask + L), ldd(mask + R));
-  dd divU = {0.f, 0.f};
-  if (DIVU) divU = duidxj[0][0] + duidxj[1][1] + duidxj[2][2];
-  const bool up = dd_gt0(mdot);
-  dd tf[3];
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    const dd uiIp = scale2(uR[i] + uL[i], 0.5f);
-    dd adv_flux;
+    dd_from_double3(gs, g[i]);
+    const dd du = dd_from_double(uR - uL), uip = scale2(dd_from_double_near(uR + uL), 0.5f);
+    // 0.5 dx . (grad u_L + grad u_R), the sum of the two sides' increments
+    const dd s = dd_dot3(hdx[0], g[i][0], hdx[1], g[i][1], hdx[2], g[i][2]);
+    corr[i] = (du - s) * inv_axdx;
     if (DEF) {
-      const dd uiUpw = up ? uL[i] + (LIMITER ? duL[i] * limitL[i] : duL[i])
-                          : uR[i] - (LIMITER ? duR[i] * limitR[i] : duR[i]);
-      adv_flux = mdot * (pecfac * uiUpw + om_pecfac * uiIp);
+      double gu[3];
+      dd gd[3];
+#pragma unroll
+      for (int j = 0; j < 3; ++j) gu[j] = up ? gl[j] : gr[j];
+      dd_from_double3(gu, gd);
+      dd t = dd_dot3(hdx[0], gd[0], hdx[1], gd[1], hdx[2], gd[2]);
+      if (LIMITER) t = t * van_leer_dd(scale2(t, 4.0f) - du, du, c.eps);
+      // upwind value - mean: u_L + t - uip = t - du / 2, or -(t - du / 2)
+      dd d = t - scale2(du, 0.5f);
+      if (!up) d = -d;
+      adv[i] = mdot * uip + mp * d;
     } else {
-      const dd uIpL = uL[i] + (LIMITER ? duL[i] * c.upw * limitL[i] : duL[i] * c.upw);
-      const dd uIpR = uR[i] - (LIMITER ? duR[i] * c.upw * limitR[i] : duR[i] * c.upw);
-      const dd uiUpw = c.alpha_upw * (up ? uIpL : uIpR) + c.om_alpha_upw * uiIp;
-      const dd uiCds = scale2(c.alpha * (uIpL + uIpR), 0.5f) + c.om_alpha * uiIp;
-      adv_flux = mdot * (pecfac * uiUpw + om_pecfac * uiCds);
+      dd gd[3];
+      dd_from_double3(gl, gd);
+      const dd duL = dd_dot3(hdx[0], gd[0], hdx[1], gd[1], hdx[2], gd[2]);
+      dd_from_double3(gr, gd);
+      const dd duR = dd_dot3(hdx[0], gd[0], hdx[1], gd[1], hdx[2], gd[2]);
+      dd tL = duL * c.upw, tR = duR * c.upw;
+      if (LIMITER) {
+        tL = tL * van_leer_dd(scale2(duL, 4.0f) - du, du, c.eps);
+        tR = tR * van_leer_dd(scale2(duR, 4.0f) - du, du, c.eps);
+      }
+      const dd uIpL = dd_from_double(uL) + tL, uIpR = dd_from_double(uR) - tR;
+      const dd uiUpw = c.alpha_upw * (up ? uIpL : uIpR) + c.om_alpha_upw * uip;
+      const dd uiCds = scale2(c.alpha * (uIpL + uIpR), 0.5f) + c.om_alpha * uip;
+      adv[i] = mdot * (pec * uiUpw + (dd{1.0f, 0.0f} - pec) * uiCds);
     }
-    const dd sd = dd_dot3(duidxj[i][0] + duidxj[0][i], av[0], duidxj[i][1] + duidxj[1][i], av[1],
-                          duidxj[i][2] + duidxj[2][i], av[2]);
-    dd diff_flux = -(viscIp * sd);
-    if (DIVU) diff_flux = divU * (c.divu_fac * viscIp * av[i]) + diff_flux;
-    tf[i] = diff_flux * maskNode + adv_flux;
   }
+  // viscous flux: -visc mask sum_j (duidxj + dujdxi) A_j
+  //   = -visc mask [corr_i |A|^2 + A_i (corr . A) + sum_j (g_ij + g_ji) A_j / 2]
+  const dd visc = scale2(dd_from_double(in.viscosity[L] + in.viscosity[R]), 0.5f);
+  const dd vm = visc * dd_min(ldd(in.mask + L), ldd(in.mask + R));
+  const dd ca = dd_dot3(corr[0], av[0], corr[1], av[1], corr[2], av[2]);
+  dd ga = ca;  // the factor of A_i
+  if (DIVU) ga = ca - c.divu_fac * (ca + scale2((g[0][0] + g[1][1]) + g[2][2], 0.5f));
+  const dd s01 = scale2(g[0][1] + g[1][0], 0.5f), s02 = scale2(g[0][2] + g[2][0], 0.5f),
+           s12 = scale2(g[1][2] + g[2][1], 0.5f);
+  dd tf[3];
+  tf[0] = adv[0] - vm * (dd_dot3(g[0][0], av[0], s01, av[1], s02, av[2]) + (corr[0] * asq + av[0] * ga));
+  tf[1] = adv[1] - vm * (dd_dot3(s01, av[0], g[1][1], av[1], s12, av[2]) + (corr[1] * asq + av[1] * ga));
+  tf[2] = adv[2] - vm * (dd_dot3(s02, av[0], s12, av[1], g[2][2], av[2]) + (corr[2] * asq + av[2] * ga));
+  // advective constants: the upwind part mdot pec of the upwind side and the
+  // central part of both
   const dd hm = scale2(mdot, 0.5f);
-  const dd habs = scale2(dd_abs(mdot), 0.5f);
-  dd aUL, aUR, aC;
+  dd x, y;
   if (DEF) {
-    aUL = (hm + habs) * pecfac;
-    aUR = (hm - habs) * pecfac;
-    aC = hm * om_pecfac;
+    const dd aC = hm - scale2(mp, 0.5f);
+    const dd w = mp + aC;
+    x = up ? aC : w;
+    y = up ? w : aC;
   } else {
-    const dd cen = c.alpha * om_pecfac * hm;
-    aUL = (hm + habs) * pecfac * c.alpha_upw + cen;
-    aUR = (hm - habs) * pecfac * c.alpha_upw + cen;
-    aC = hm * (pecfac * c.om_alpha_upw + om_pecfac * c.om_alpha);
+    const dd om_pec = dd{1.0f, 0.0f} - pec;
+    const dd cen = c.alpha * om_pec * hm + hm * (pec * c.om_alpha_upw + om_pec * c.om_alpha);
+    const dd ua = mp * c.alpha_upw;
+    x = up ? cen : ua + cen;
+    y = up ? ua + cen : cen;
   }
-  const dd t = -(viscIp * inv_axdx);
-  const dd dlhsfac = t * asq;
+  const dd t = -(visc * inv_axdx);
+  const dd dl = t * asq;
   const dd ta0 = t * av[0], ta1 = t * av[1], ta2 = t * av[2];
-  b[0] = (aUR + aC) + dlhsfac;
-  b[E] = (-aUL - aC) + dlhsfac;
-  b[2 * E] = ta0 * av[0];
-  b[3 * E] = ta0 * av[1];
-  b[4 * E] = ta0 * av[2];
-  b[5 * E] = ta1 * av[1];
-  b[6 * E] = ta1 * av[2];
-  b[7 * E] = ta2 * av[2];
-  b[8 * E] = tf[0];
-  b[9 * E] = tf[1];
-  b[10 * E] = tf[2];
+  const double cLR = dd_to_double_int(x + dl), cRL = dd_to_double_int(dl - y);
+  const double n00 = dd_to_double_int(ta0 * av[0]), n11 = dd_to_double_int(ta1 * av[1]),
+               n22 = dd_to_double_int(ta2 * av[2]);
+  st32(rec, n00 + cLR, n00 + cRL, pair_bits(tf[0]), dd_to_double_int(ta0 * av[1]));
+  st32(rec + 4, n11 + cLR, n11 + cRL, pair_bits(tf[1]), dd_to_double_int(ta1 * av[2]));
+  st32(rec + 8, n22 + cLR, n22 + cRL, pair_bits(tf[2]), dd_to_double_int(ta0 * av[2]));
 }
 
 template <bool LIMITER, bool DIVU, bool DEF>
 __global__ void __launch_bounds__(kThreads, 4)
-    momentum_edge_k(int64_t E, int64_t e0, int64_t e1, MomentumIn in, MomentumDD c,
-                    dd* __restrict__ buf) {
+    momentum_edge_k(int64_t e0, int64_t e1, MomentumIn in, MomentumDD c, double* __restrict__ buf) {
   const int64_t e = e0 + int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (e >= e1) return;
-  momentum_edge<LIMITER, DIVU, DEF>(e, E, in, c, buf + e);
+  momentum_edge<LIMITER, DIVU, DEF>(e, in, c, buf + kMomentumCoefs * e);
 }
 
 // ---------------------------------------------------------------------------
@@ -573,141 +588,218 @@ __global__ void __launch_bounds__(kRow1Threads)
     values[base + k] = accumulate ? values[base + k] + stage[k] : stage[k];
 }
 
-// 3-dof momentum, one thread per CSR row (three per node row, dof q =
-// thread % 3): each thread accumulates its row of every 3x3 block from the
-// float-pair coefficients and widens it to FP64 with integer operations
-// (dd_to_double_int: no FP64 instruction per entry); a block of kRow3Nodes node
-// rows stages their CSR range in shared memory and writes it coalesced.
-// (One thread per node row, with the symmetric blocks widened once, needs
-// a third fewer FP64 adds but ran at a third of the occupancy: the shared
-// staging per node is the same, so measured 0.357 against 0.328 ms.)
-// Off-diagonal block of an incident edge: c_side I + N; diagonal block:
-// -(sum of the other side's constants + sum of N) / relax.
-constexpr int kRow3Nodes = 64;
+// 3-dof momentum, one thread per CSR row (three neighbouring lanes per node
+// row, ten nodes a warp) over the row's incident edges in column order.
+// Off-diagonal entries are copied from the edge's record; the diagonal block
+// -(sum of the opposite D e_q + sum of N)_q / relax is summed in FP64, the rhs
+// in float pairs. Thread q loads sector q of a record with one 32-byte load
+// (a record is one line and a warp's ten records eleven or so, where eight-
+// byte loads of the same words cost five times the L1 lookups), sums its own
+// entry of N and takes the other one it stores from the node's next lane.
+// The next record is loaded while one is summed. A warp stages its CSR range in
+// shared memory and writes it with one bulk copy. What it reads and writes (96
+// bytes an edge, the matrix) takes 125 us at 128 x 128 x 64; it takes 172,
+// with FP64 pipe, issue and L1 each about half busy (24 warps a SM without
+// spills measured the same as 36 with).
+constexpr int kRow3Warps = 6, kRow3PerSm = 4;
+constexpr int kRow3Group = 10;  // node rows of a warp, three lanes each
 struct Row3Args {
-  int64_t R, E;  // end of the node rows; stride of the coefficient arrays
+  int64_t R;  // end of the node rows
   int64_t r_begin;  // first node row (the row kernel's blocks start here)
-  int64_t mask;  // edge -> coefficient slot: e & mask
+  int64_t mask;  // edge -> record: e & mask
   const int32_t* __restrict__ inc_ptr;
   const uint32_t* __restrict__ inc;
   const int32_t* __restrict__ diag_pos;
   const int64_t* __restrict__ row_ptr;
-  const dd* cb;  // not restrict: the single-kernel assembly writes it in flight
-  dd irelax;
+  const double* rec;  // not restrict: the single-kernel assembly writes it in flight
+  double irelax;
   double* __restrict__ values;
   double* __restrict__ rhs;
   int accumulate, smem_bytes;
 };
 
-// coefficient loads: through the read-only path when the buffer is not
-// written during the kernel (NC), else plain loads
+// one sector of a record: through the read-only path when the buffer is not
+// written during the kernel (NC), else a plain load
 template <bool NC>
-__device__ __forceinline__ dd ldc(const dd* p) {
-  if constexpr (NC) {
-    const float2 v = __ldg(reinterpret_cast<const float2*>(p));
-    return {v.x, v.y};
-  } else {
-    return *p;
-  }
+__device__ __forceinline__ void ld32(const double* p, double (&x)[4]) {
+  if constexpr (NC)
+    asm volatile("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+                 : "=d"(x[0]), "=d"(x[1]), "=d"(x[2]), "=d"(x[3])
+                 : "l"(p));
+  else
+    asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+                 : "=d"(x[0]), "=d"(x[1]), "=d"(x[2]), "=d"(x[3])
+                 : "l"(p)
+                 : "memory");
 }
 
-// One block of NB node rows starting at r0 (threads 0 .. 3 NB - 1 of the
-// block; any others only take part in the staging copy).
-// IDX: the type of the coefficient offsets (uint32_t when 11 E < 2^31:
-// one register and one wide multiply-add per load instead of a 64-bit
-// pointer per coefficient array). ACC: 0 overwrite, 1 add to the values
-// present, -1 as a.accumulate says (the write mode as a constant drops the
-// read and select of every store).
-template <int NB, bool NC, typename IDX = int64_t, int ACC = -1>
-__device__ __forceinline__ void row3_block(int64_t r0, const Row3Args& a, double* stage) {
-  const dd* cb = a.cb;
+// *p += x with an addition that stays inside its branch
+__device__ __forceinline__ void add64(double* p, double x) {
+  double y = *p;
+  asm volatile("add.f64 %0, %0, %1;" : "+d"(y) : "d"(x));
+  *p = y;
+}
+
+// Bulk copy of `bytes` (a multiple of 16) from shared to global memory, both
+// 16-byte aligned, by one thread after the others' writes have been fenced
+// (fence_async) and joined.
+__device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+__device__ __forceinline__ void bulk_store(double* dst, const double* src, int bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst),
+               "r"(uint32_t(__cvta_generic_to_shared(src))), "r"(bytes)
+               : "memory");
+  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+// the calling thread's bulk copies have read their sources
+__device__ __forceinline__ void bulk_wait() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+
+// Groups g, g + step, ... of kRow3Group node rows from row `first` to `end`,
+// by one warp, which stages each group's CSR range and writes it: no block
+// barrier. A group starts with a chain of loads (list bounds, list, record),
+// as long as the sums themselves at the matrix sizes here, so the next
+// group's bounds are loaded with this group's records and its first record
+// while this group's rows are finished.
+// IDX: the type of the record offsets (uint32_t when 12 E < 2^31: one
+// register and one wide multiply-add per record instead of 64-bit
+// arithmetic). ACC: 0 overwrite, 1 add to the values present, -1 as
+// a.accumulate says (the write mode as a constant drops the read and select
+// of every store).
+template <bool NC, typename IDX = int64_t, int ACC = -1>
+__device__ __forceinline__ void row3_groups(int64_t g, int64_t step, int64_t first, int64_t end_row,
+                                            const Row3Args& a, double* stage) {
   const bool accumulate = ACC < 0 ? a.accumulate != 0 : ACC != 0;
-  const IDX E = IDX(a.E);
-  const int64_t mask = a.mask;
-  const int64_t r1 = (r0 + NB < a.R) ? r0 + NB : a.R;
-  const int64_t base = a.row_ptr[3 * r0];
-  const int64_t cnt = a.row_ptr[3 * r1] - base;
-  const bool staged = cnt * int64_t(sizeof(double)) <= a.smem_bytes;
-  const int local = threadIdx.x / 3, q = threadIdx.x - 3 * (threadIdx.x / 3);
-  const int64_t r = local < NB ? r0 + local : r1;
-  // row q of the symmetric N (N00 N01 N02 N11 N12 N22 at slots 2..7): its
-  // diagonal N_qq and the off-diagonals of columns c1 < c2 (the two c != q),
-  // so that the block's c_side I term adds to one fixed entry
-  const int c1 = q == 0 ? 1 : 0, c2 = q == 2 ? 1 : 2;
-  const IDX xd = IDX(q == 0 ? 2 : (q == 1 ? 5 : 7)) * E;
-  const IDX x1 = IDX(q == 2 ? 4 : 3) * E;
-  const IDX x2 = IDX(q == 0 ? 4 : 6) * E;
-  const IDX xf = IDX(8 + q) * E;
-  if (r < r1) {
-    const int32_t s = a.inc_ptr[r], t = a.inc_ptr[r + 1];
-    const int64_t bq = a.row_ptr[3 * r + q];
-    double* v = staged ? stage + (bq - base) : a.values + bq;
+  const int lane = threadIdx.x & 31, trio = lane / 3, q = lane - 3 * trio;
+  const int next = 3 * trio + (q + 2) % 3;  // the lane that holds the other entry of N
+  // columns of thread q's own entry of N (0: N01, 1: N12, 2: N02) and of the
+  // other one (0: N02, 1: N01, 2: N12)
+  const int cn = q == 0 ? 1 : (q == 1 ? 2 : 0), co = q == 0 ? 2 : (q == 1 ? 0 : 1);
+  struct Bounds {
+    int64_t base, bq;  // CSR position of the group and of this lane's row
+    int32_t s, t, cnt, dp;
+  };
+  auto bounds = [&](int64_t gr) {
+    Bounds b{0, 0, 0, 0, 0, 0};
+    const int64_t r0 = first + gr * kRow3Group;
+    if (r0 >= end_row) return b;
+    const int64_t r1 = r0 + kRow3Group < end_row ? r0 + kRow3Group : end_row, r = r0 + trio;
+    b.base = a.row_ptr[3 * r0];
+    b.cnt = int32_t(a.row_ptr[3 * r1] - b.base);
+    if (trio < kRow3Group && r < r1) {
+      b.s = a.inc_ptr[r];
+      b.t = a.inc_ptr[r + 1];
+      b.bq = a.row_ptr[3 * r + q];
+      b.dp = a.diag_pos[r];
+    }
+    return b;
+  };
+  auto load = [&](uint32_t w, double (&x)[4]) {
+    ld32<NC>(a.rec + IDX(kMomentumCoefs) * IDX(int64_t((w & 0x7fffffffu) >> 1) & a.mask) + 4 * q, x);
+  };
+  if (first + g * kRow3Group >= end_row) return;
+  Bounds b = bounds(g);
+  uint32_t w = b.s < b.t ? a.inc[b.s] : 0u, wn = b.s + 1 < b.t ? a.inc[b.s + 1] : 0u;
+  double x[4];
+  if (b.s < b.t) load(w, x);
+  for (;;) {
+    const int64_t r = first + g * kRow3Group + trio;
+    g += step;
+    const Bounds bn = bounds(g);
+    if (lane == 0) bulk_wait();  // the previous group's copy has left the stage
+    __syncwarp();
+    const int s = b.s, t = b.t, dp = b.dp;
+    // the staged range keeps the parity of the CSR position, so that both
+    // sides of the copy are 16-byte aligned together
+    const int odd = int(b.base & 1);
+    const bool staged = (b.cnt + odd) * int(sizeof(double)) <= a.smem_bytes;
     const bool acc = accumulate && !staged;
-    if (s != t) {
-      const int dp = a.diag_pos[r];
-      // sums over the incident edges: the diagonal entry's N_qq + c_other,
-      // the two off-diagonal N sums and the rhs (deferred renormalisation)
-      dd_acc sdg, s1, s2, rr;
-      dd od{}, o1{}, o2{};
-      int slot = -1;
-      auto put3 = [&](int k, dd xd, dd x1, dd x2) {
-        const double d0 = dd_to_double_int(xd), d1 = dd_to_double_int(x1),
-                     d2 = dd_to_double_int(x2);
-        v[k + q] = acc ? v[k + q] + d0 : d0;
-        v[k + c1] = acc ? v[k + c1] + d1 : d1;
-        v[k + c2] = acc ? v[k + c2] + d2 : d2;
-      };
-      for (int32_t qi = s; qi < t; ++qi) {
-        const uint32_t w = a.inc[qi];
-        const bool dup = (w >> 31) != 0;
-        const IDX e = IDX(int64_t((w & 0x7fffffffu) >> 1) & mask);
-        const int side = w & 1u;
-        const dd c0 = ldc<NC>(cb + e), c1v = ldc<NC>(cb + (E + e));
-        const dd co = side ? c1v : c0, other = side ? c0 : c1v;
-        const dd nd = ldc<NC>(cb + (xd + e)), n1 = ldc<NC>(cb + (x1 + e)), n2 = ldc<NC>(cb + (x2 + e));
-        const dd f = ldc<NC>(cb + (xf + e));
-        acc_add(rr, side ? f : -f);
-        const dd bd = nd + co;
-        if (!dup) {
-          if (slot >= 0) put3(3 * (slot < dp ? slot : slot + 1), od, o1, o2);
-          ++slot;
-          od = bd;
-          o1 = n1;
-          o2 = n2;
-        } else {
-          od = od + bd;
-          o1 = o1 + n1;
-          o2 = o2 + n2;
-        }
-        acc_add(sdg, nd);
-        acc_add(sdg, other);
-        acc_add(s1, n1);
-        acc_add(s2, n2);
-      }
-      put3(3 * (slot < dp ? slot : slot + 1), od, o1, o2);
-      // diagonal block row q: -(sum(other) e_q + sum(N)_q) / relax
-      put3(3 * dp, -(acc_value(sdg) * a.irelax), -(acc_value(s1) * a.irelax),
-           -(acc_value(s2) * a.irelax));
-      const double d = dd_to_double_int(acc_value(rr));
-      a.rhs[3 * r + q] = accumulate ? a.rhs[3 * r + q] + d : d;
-    } else if (!acc) {
-      for (int64_t k = 0; k < a.row_ptr[3 * r + q + 1] - bq; ++k) v[k] = 0.0;
+    double* v = staged ? stage + odd + (b.bq - b.base) : a.values + b.bq;
+    if (s == t && trio < kRow3Group && r < end_row && !acc) {
+      const int64_t len = a.row_ptr[3 * r + q + 1] - b.bq;
+      for (int64_t k = 0; k < len; ++k) v[k] = 0.0;
       if (!accumulate) a.rhs[3 * r + q] = 0.0;
     }
+    auto put3 = [&](int k, double d, double n, double o) {
+      v[k + q] = acc ? v[k + q] + d : d;
+      v[k + cn] = acc ? v[k + cn] + n : n;
+      v[k + co] = acc ? v[k + co] + o : o;
+    };
+    dd_acc rr;
+    double sd = 0.0, sn = 0.0;
+    int slot = -1;
+    // every lane takes the warp's largest number of rounds (the exchange is
+    // warp-wide); the next record and the incidence after it are in flight
+    // while a record is summed (two records ahead measured the same)
+    const int most = __reduce_max_sync(0xffffffffu, t - s);
+#pragma unroll 2
+    for (int k = 0; k < most; ++k) {
+      double xn[4];
+      if (s + k + 1 < t) load(wn, xn);
+      const uint32_t w2 = s + k + 2 < t ? a.inc[s + k + 2] : 0u;
+      const double other = __shfl_sync(0xffffffffu, x[3], next);
+      if (s + k < t) {
+        const bool side = (w & 1u) != 0, dup = (w >> 31) != 0;
+        const double own = side ? x[1] : x[0], opp = side ? x[0] : x[1];
+        const dd f{__int_as_float(__double2loint(x[2])), __int_as_float(__double2hiint(x[2]))};
+        acc_add(rr, side ? f : -f);
+        slot += dup ? 0 : 1;
+        const int col = 3 * (slot < dp ? slot : slot + 1);
+        if (!dup) {
+          put3(col, own, x[3], other);
+        } else {  // a repeated column (periodic pairs)
+          add64(v + col + q, own);
+          add64(v + col + cn, x[3]);
+          add64(v + col + co, other);
+        }
+        sd += opp;
+        sn += x[3];
+      }
+      w = wn;
+      wn = w2;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) x[j] = xn[j];
+    }
+    // the next group's first incidences, then its first record
+    const bool more = bn.s < bn.t;
+    w = more ? a.inc[bn.s] : 0u;
+    wn = bn.s + 1 < bn.t ? a.inc[bn.s + 1] : 0u;
+    const double so = __shfl_sync(0xffffffffu, sn, next);
+    if (s != t) {
+      put3(3 * dp, -sd * a.irelax, -sn * a.irelax, -so * a.irelax);
+      const double d = dd_to_double_int(acc_value(rr));
+      a.rhs[3 * r + q] = accumulate ? a.rhs[3 * r + q] + d : d;
+    }
+    if (more) load(w, x);
+    if (staged) {
+      double* out = a.values + b.base - odd;
+      const int end = b.cnt + odd;
+      if (!accumulate) {
+        // the whole 16-byte pairs as one bulk copy, the ends by hand
+        fence_async();
+        __syncwarp();
+        if (lane == 1 && odd && end > 1) out[1] = stage[1];
+        if (lane == 2 && (end & 1) && end > odd) out[end - 1] = stage[end - 1];
+        const int from = 2 * odd, bytes = ((end & ~1) - from) * int(sizeof(double));
+        if (lane == 0 && bytes > 0) bulk_store(out + from, stage + from, bytes);
+      } else {
+        __syncwarp();
+        for (int k = odd + lane; k < end; k += 32) out[k] += stage[k];
+        __syncwarp();
+      }
+    }
+    if (first + g * kRow3Group >= end_row) {
+      if (lane == 0) bulk_wait();
+      return;
+    }
+    b = bn;
   }
-  if (!staged) return;
-  __syncthreads();
-  // a staged range fits the shared array: 32-bit counts
-  double* out = a.values + base;
-  const int n = int(cnt);
-  for (int k = int(threadIdx.x); k < n; k += int(blockDim.x))
-    out[k] = accumulate ? out[k] + stage[k] : stage[k];
 }
 
 template <typename IDX, int ACC>
-__global__ void __launch_bounds__(3 * kRow3Nodes) row3t_k(Row3Args a) {
+__global__ void __launch_bounds__(32 * kRow3Warps, kRow3PerSm) row3t_k(Row3Args a) {
   extern __shared__ double stage[];
-  row3_block<kRow3Nodes, true, IDX, ACC>(a.r_begin + int64_t(blockIdx.x) * kRow3Nodes, a, stage);
+  row3_groups<true, IDX, ACC>(int64_t(blockIdx.x) * kRow3Warps + (threadIdx.x >> 5),
+                              int64_t(gridDim.x) * kRow3Warps, a.r_begin, a.R, a,
+                              stage + (threadIdx.x >> 5) * (a.smem_bytes >> 3));
 }
 
 // ---------------------------------------------------------------------------
@@ -779,7 +871,7 @@ __device__ bool wait_flags(const int* flags, const int32_t* list, int n, int gen
 
 template <bool LIMITER, bool DIVU, bool DEF>
 __global__ void __launch_bounds__(kFusedChunk, 4)
-    momentum_fused_k(FusedArgs f, MomentumIn in, MomentumDD c, Row3Args ra, dd* ring) {
+    momentum_fused_k(FusedArgs f, MomentumIn in, MomentumDD c, Row3Args ra, double* ring) {
   extern __shared__ double stage[];
   __shared__ int s_item[2];
   int next = 0;
@@ -797,7 +889,9 @@ __global__ void __launch_bounds__(kFusedChunk, 4)
     if (it & 1) {
       const int b = f.in_ptr[idx];
       if (wait_flags(f.eflag, f.in + b, f.in_ptr[idx + 1] - b, f.gen, f.err))
-        row3_block<kFusedBlock, false>(int64_t(idx) * kFusedBlock, ra, stage);
+        row3_groups<false>(threadIdx.x >> 5, kFusedBlock / kRow3Group, int64_t(idx) * kFusedBlock,
+                           min(int64_t(idx + 1) * kFusedBlock, ra.R), ra,
+                           stage + (threadIdx.x >> 5) * (ra.smem_bytes >> 3));
       __syncthreads();
       if (threadIdx.x == 0) st_release(f.rflag + idx, f.gen);
     } else {
@@ -806,7 +900,7 @@ __global__ void __launch_bounds__(kFusedChunk, 4)
       const bool ok = prev < 0 || wait_flags(f.rflag, f.out + f.out_ptr[prev],
                                              f.out_ptr[prev + 1] - f.out_ptr[prev], f.gen, f.err);
       const int64_t e = int64_t(idx) * kFusedChunk + threadIdx.x;
-      if (ok && e < f.num_edges) momentum_edge<LIMITER, DIVU, DEF>(e, ra.E, in, c, ring + (e & ra.mask));
+      if (ok && e < f.num_edges) momentum_edge<LIMITER, DIVU, DEF>(e, in, c, ring + kMomentumCoefs * (e & ra.mask));
       __syncthreads();
       if (threadIdx.x == 0) st_release(f.eflag + idx, f.gen);
     }
@@ -868,11 +962,12 @@ inline unsigned grid_for(int64_t n, int t = kThreads) {
   return unsigned((n + t - 1) / t);
 }
 
-int g_smem_set_device = -1;
+int g_smem_set_device = -1, g_sms = 1;
 void set_smem_attrs() {
   int dev = 0;
   NW_CUDA(cudaGetDevice(&dev));
   if (g_smem_set_device == dev) return;
+  NW_CUDA(cudaDeviceGetAttribute(&g_sms, cudaDevAttrMultiProcessorCount, dev));
   NW_CUDA(cudaFuncSetAttribute(row1_k<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxRowSmem));
   NW_CUDA(cudaFuncSetAttribute(row1_k<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxRowSmem));
   NW_CUDA(cudaFuncSetAttribute(row3t_k<uint32_t, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxRowSmem));
@@ -965,7 +1060,6 @@ MomentumDD momentum_dd(const MomentumOpts& o) {
   c.om_alpha_upw = dd_param(1.0 - o.alpha_upw);
   c.upw = dd_param(o.upw_factor);
   c.divu_fac = dd_param(2.0 / 3.0 * o.include_div_u);
-  c.irelax = dd_param(1.0 / o.relax);
   c.eps = dd_param(1.0e-16);
   return c;
 }
@@ -973,24 +1067,23 @@ MomentumIn momentum_in(const int2* edges, const nw_momentum_fields& f) {
   return MomentumIn{edges, f.coords, f.velocity, f.dudx, f.viscosity, f.mask, f.area, f.mdot, f.pecfac};
 }
 Row3Args row3_args(int64_t R, const int32_t* inc_ptr, const uint32_t* inc, const int32_t* diag_pos,
-                   const int64_t* row_ptr, const double* buf, int64_t E, double relax, double* values,
+                   const int64_t* row_ptr, const double* buf, double relax, double* values,
                    double* rhs, int accumulate, int smem_bytes) {
-  return Row3Args{R, E, 0, int64_t(-1), inc_ptr, inc, diag_pos, row_ptr, reinterpret_cast<const dd*>(buf),
-                  dd_param(1.0 / relax), values, rhs, accumulate, smem_bytes};
+  return Row3Args{R, 0, int64_t(-1), inc_ptr, inc, diag_pos, row_ptr, buf, 1.0 / relax, values, rhs,
+                  accumulate, smem_bytes};
 }
 }  // namespace
 
-void launch_momentum_edges(cudaStream_t s, int64_t E, int64_t e0, int64_t e1, const int2* edges,
+void launch_momentum_edges(cudaStream_t s, int64_t e0, int64_t e1, const int2* edges,
                            const nw_momentum_fields& f, const MomentumOpts& o,
                            double* buf) {
   if (e1 <= e0) return;
   const MomentumDD c = momentum_dd(o);
   const MomentumIn in = momentum_in(edges, f);
-  dd* b = reinterpret_cast<dd*>(buf);
   const bool lim = o.use_limiter != 0, divu = o.include_div_u != 0.0;
   const bool def = o.alpha == 0.0 && o.alpha_upw == 1.0 && o.upw_factor == 1.0;
 #define NW_MOM(LIM, DIV, DEF) \
-  momentum_edge_k<LIM, DIV, DEF><<<grid_for(e1 - e0), kThreads, 0, s>>>(E, e0, e1, in, c, b)
+  momentum_edge_k<LIM, DIV, DEF><<<grid_for(e1 - e0), kThreads, 0, s>>>(e0, e1, in, c, buf)
 #define NW_MOM2(LIM, DIV) \
   if (def) NW_MOM(LIM, DIV, true); \
   else NW_MOM(LIM, DIV, false)
@@ -1006,7 +1099,7 @@ int fused_blocks_per_sm(int smem_bytes) {
   set_smem_attrs();
   int occ = 0;
   NW_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, momentum_fused_k<false, false, true>,
-                                                        kFusedChunk, smem_bytes));
+                                                        kFusedChunk, smem_bytes * (kFusedChunk / 32)));
   return occ;
 }
 
@@ -1016,17 +1109,16 @@ void launch_momentum_fused(cudaStream_t s, const FusedLaunch& L, const int2* edg
   set_smem_attrs();
   const MomentumDD c = momentum_dd(o);
   const MomentumIn in = momentum_in(edges, f);
-  Row3Args ra = row3_args(L.R, L.inc_ptr, L.inc, L.diag_pos, L.row_ptr, L.ring, L.stride, o.relax,
-                          L.values, L.rhs, L.accumulate, L.smem_bytes);
+  Row3Args ra = row3_args(L.R, L.inc_ptr, L.inc, L.diag_pos, L.row_ptr, L.ring, o.relax, L.values, L.rhs,
+                          L.accumulate, L.smem_bytes);
   ra.mask = L.mask;
   FusedArgs fa{L.items, L.in_ptr, L.in, L.out_ptr, L.out, L.eflag, L.rflag,
                L.ticket, L.err, L.num_edges, L.ring_chunks, int(L.nitems), L.gen};
-  dd* ring = reinterpret_cast<dd*>(L.ring);
   NW_CUDA(cudaMemsetAsync(L.ticket, 0, sizeof(int), s));
   const bool lim = o.use_limiter != 0, divu = o.include_div_u != 0.0;
   const bool def = o.alpha == 0.0 && o.alpha_upw == 1.0 && o.upw_factor == 1.0;
 #define NW_FUSED(LIM, DIV, DEF) \
-  momentum_fused_k<LIM, DIV, DEF><<<L.grid, kFusedChunk, L.smem_bytes, s>>>(fa, in, c, ra, ring)
+  momentum_fused_k<LIM, DIV, DEF><<<L.grid, kFusedChunk, L.smem_bytes * (kFusedChunk / 32), s>>>(fa, in, c, ra, L.ring)
 #define NW_FUSED2(LIM, DIV) \
   if (def) NW_FUSED(LIM, DIV, true); \
   else NW_FUSED(LIM, DIV, false)
@@ -1038,7 +1130,7 @@ void launch_momentum_fused(cudaStream_t s, const FusedLaunch& L, const int2* edg
 #undef NW_FUSED
 }
 
-int row_block_nodes(int kind) { return kind == 3 ? kFusedBlock : (kind == 2 ? kRow3Nodes : kRow1Threads); }
+int row_block_nodes(int kind) { return kind >= 2 ? kRow3Group : kRow1Threads; }
 
 int row_stage_bytes(int kind, const int64_t* row_ptr_host, int64_t R) {
   const int nb = row_block_nodes(kind);
@@ -1048,6 +1140,12 @@ int row_stage_bytes(int kind, const int64_t* row_ptr_host, int64_t R) {
     const int64_t r1 = r0 + nb < R ? r0 + nb : R;
     const int64_t c = row_ptr_host[nd * r1] - row_ptr_host[nd * r0];
     if (c > mx) mx = c;
+  }
+  // kind 2 and 3: bytes of one warp, one more entry so that the range can
+  // start at its parity, a multiple of 16
+  if (kind >= 2) {
+    const int64_t most = kMaxRowSmem / (kFusedChunk / 32);
+    return int(std::min<int64_t>((mx + 2) / 2 * 16, most));
   }
   const int64_t bytes = mx * int64_t(sizeof(double));
   return bytes <= kMaxRowSmem ? int(bytes) : kMaxRowSmem;
@@ -1067,19 +1165,21 @@ void launch_rows(cudaStream_t s, int kind, int64_t R, const int32_t* inc_ptr,
     row1_k<1><<<grid_for(R, kRow1Threads), kRow1Threads, smem_bytes, s>>>(
         R, inc_ptr, inc, diag_pos, row_ptr, buf, E, values, rhs, accumulate, smem_bytes);
   else {
-    Row3Args a = row3_args(R, inc_ptr, inc, diag_pos, row_ptr, buf, E, relax, values, rhs,
-                           accumulate, smem_bytes);
+    Row3Args a = row3_args(R, inc_ptr, inc, diag_pos, row_ptr, buf, relax, values, rhs, accumulate, smem_bytes);
     a.r_begin = row_begin;
-    const unsigned grid = grid_for(R - row_begin, kRow3Nodes);
+    // one wave of blocks: registers allow kRow3PerSm a SM, the staging fewer
+    const int smem = smem_bytes * kRow3Warps;
+    const int occ = std::max(1, std::min(kRow3PerSm, kSmSmem / (smem + 1024)));
+    const unsigned grid = std::min(grid_for(R - row_begin, kRow3Group * kRow3Warps), unsigned(occ * g_sms));
     const bool narrow = int64_t(kMomentumCoefs) * E < (int64_t(1) << 31);
     if (narrow && !accumulate)
-      row3t_k<uint32_t, 0><<<grid, 3 * kRow3Nodes, smem_bytes, s>>>(a);
+      row3t_k<uint32_t, 0><<<grid, 32 * kRow3Warps, smem, s>>>(a);
     else if (narrow)
-      row3t_k<uint32_t, 1><<<grid, 3 * kRow3Nodes, smem_bytes, s>>>(a);
+      row3t_k<uint32_t, 1><<<grid, 32 * kRow3Warps, smem, s>>>(a);
     else if (!accumulate)
-      row3t_k<int64_t, 0><<<grid, 3 * kRow3Nodes, smem_bytes, s>>>(a);
+      row3t_k<int64_t, 0><<<grid, 32 * kRow3Warps, smem, s>>>(a);
     else
-      row3t_k<int64_t, 1><<<grid, 3 * kRow3Nodes, smem_bytes, s>>>(a);
+      row3t_k<int64_t, 1><<<grid, 32 * kRow3Warps, smem, s>>>(a);
   }
 }
 

@@ -14,10 +14,11 @@ using MomentumOpts = nw_momentum_opts;
 
 // 8-byte coefficient slots per edge written by the edge phase: scalar, six
 // FP64 SoA arrays of E; continuity, one 16-byte record (f, tmdot as float
-// pairs) per edge; momentum, 11 SoA arrays of E float pairs.
+// pairs) per edge; momentum, one 96-byte record per edge (nine FP64 CSR
+// entries and three float pairs, see momentum_edge).
 constexpr int kScalarCoefs = 6;
 constexpr int kContinuityCoefs = 2;
-constexpr int kMomentumCoefs = 11;
+constexpr int kMomentumCoefs = 12;
 
 void launch_scalar_edges(cudaStream_t s, int64_t E, const int2* edges,
                          const nw_scalar_fields& f, const ScalarOpts& o,
@@ -38,9 +39,9 @@ void launch_continuity_edge_range(cudaStream_t s, int64_t n0, int64_t n1, int64_
                                   const int2* edges, const nw_continuity_fields& f,
                                   const ContinuityOpts& o, double* buf, double* nodebuf);
 constexpr int kContinuityNodeStride = 8;
-// Edge phase of the momentum assembly over edges [e0, e1) of E (the
-// coefficient buffer is laid out with stride E).
-void launch_momentum_edges(cudaStream_t s, int64_t E, int64_t e0, int64_t e1, const int2* edges,
+// Edge phase of the momentum assembly over edges [e0, e1): record e of the
+// buffer.
+void launch_momentum_edges(cudaStream_t s, int64_t e0, int64_t e1, const int2* edges,
                            const nw_momentum_fields& f, const MomentumOpts& o,
                            double* buf);
 // kind 0 scalar, 1 continuity, 2 momentum (3 dof), over node rows
@@ -55,8 +56,7 @@ void launch_rows(cudaStream_t s, int kind, int64_t R, const int32_t* inc_ptr,
 int row_stage_bytes(int kind, const int64_t* row_ptr_host, int64_t R);
 
 // Single-kernel momentum assembly (momentum_fused_k) over the work list of
-// schedule.h. ring: the coefficient slots (stride `stride`, edge e in slot
-// e & mask); eflag / rflag: one flag per edge chunk / row block, never
+// schedule.h. ring: the edge records (edge e in slot e & mask); eflag / rflag: one flag per edge chunk / row block, never
 // reset (a launch waits for its own generation `gen`); ticket: the work
 // counter (cleared by the launch); err: set to 1 when a wait timed out.
 struct FusedLaunch {

@@ -10,7 +10,7 @@
 //   add:  |err| <= 2 u^2 (|a| + |b|)      (relative to the operand sizes,
 //                                          not to the possibly cancelling sum)
 //   mul:  |err| <= 4 u^2 |a b|
-//   rcp:  |err| <= 3 u^2 / |x|            (one Newton step from a float seed)
+//   rcp:  |err| <= 3 u^2 / |x|            (a quadratic step from a float seed)
 // Conversions from double keep the top 48 significand bits (the split error
 // is <= 2^-48 relative); dd -> double rounds hi + lo once. The
 // exponent range is the float range: |x| >= 2^128 becomes infinite, and
@@ -192,24 +192,92 @@ NW_HD double dd_to_double_int(dd a) {
 // Split of a double into hi (top 24 significand bits) + lo (the next 24,
 // rounded), with integer operations for |x| in [2^-62, 2^127); zeros are
 // exact; anything else takes the conversion instructions.
-NW_HD dd dd_from_double(double x) {
+//
+// In that range hi's bits are the double's shifted left by three, its low
+// eight exponent bits rebiased by -896 = 128 (mod 256), i.e. with bit 7
+// flipped. The remaining 29 bits are worth rest * 2^(ex - 1075): a float of
+// hi's exponent field less 52. |lo| < ulp(hi): the pair is used as it is (the
+// double-word operations only need |lo| below ulp(hi), not a rounded split).
+NW_HD uint32_t dd_split_range(uint32_t hw) { return hw * 2u - (961u << 21); }  // in range: below kDdSplit
+constexpr uint32_t kDdSplit = 189u << 21;
+NW_HD dd dd_split_bits(uint32_t hw, uint32_t lw) {
+#ifdef __CUDA_ARCH__
+  const uint32_t f = __funnelshift_l(lw, hw, 3);
+#else
+  const uint32_t f = (hw << 3) | (lw >> 29);
+#endif
+  const uint32_t hi = ((f ^ 0x40000000u) & 0x7fffffffu) | (hw & 0x80000000u);
+  const float rest = float(lw & 0x1fffffffu);  // exact up to 2^24, rounded above
+  return {u2f(hi), fmul(rest, u2f((hi & 0xff800000u) - (52u << 23)))};
+}
+// the same with hi rounded to nearest, so that |lo| <= ulp(hi) / 2 and the
+// pair holds one more bit of x: 2^28 is added before hi is cut, and lo is the
+// signed remainder
+NW_HD dd dd_split_near(uint32_t hw, uint32_t lw) {
+  const uint64_t b = ((uint64_t(hw) << 32) | lw) + 0x10000000u;
+  const uint32_t h = uint32_t(b >> 32);
+#ifdef __CUDA_ARCH__
+  const uint32_t f = __funnelshift_l(uint32_t(b), h, 3);
+#else
+  const uint32_t f = (h << 3) | (uint32_t(b) >> 29);
+#endif
+  const uint32_t hi = ((f ^ 0x40000000u) & 0x7fffffffu) | (hw & 0x80000000u);
+  const float rest = float(int32_t(lw << 3));  // 8 times the remainder
+  const uint32_t e = (((hw << 3) ^ 0x40000000u) & 0x7f800000u) | (hw & 0x80000000u);  // x's own exponent
+  return {u2f(hi), fmul(rest, u2f(e - (55u << 23)))};
+}
+// zeros and everything outside that range, kept out of line on the device
+#ifdef __CUDACC__
+__host__ __device__ __noinline__ inline
+#else
+inline
+#endif
+dd dd_from_double_slow(double x) {
   const uint64_t b = d2u(x);
-  const uint32_t hw = uint32_t(b >> 32), lw = uint32_t(b);
-  const int ex = int((hw >> 20) & 0x7ffu);
-  const uint32_t sign = hw & 0x80000000u;
-  if (ex >= 961 && ex < 1150) {
-    const float hi = u2f(sign | (uint32_t(ex - 896) << 23) | ((hw & 0xfffffu) << 3) | (lw >> 29));
-    // the remaining 29 bits are worth rest * 2^(ex - 1075)
-    const float rest = float(lw & 0x1fffffffu);  // exact up to 2^24, rounded above
-    const float scale = u2f(uint32_t(ex - 1075 + 127) << 23);
-    // |lo| < ulp(hi): the pair is used as it is (the double-word
-    // operations only need |lo| below ulp(hi), not a rounded split)
-    return {hi, u2f(f2u(fmul(rest, scale)) | sign)};
-  }
-  if ((b << 1) == 0) return {u2f(sign), 0.0f};
+  if ((b << 1) == 0) return {u2f(uint32_t(b >> 32) & 0x80000000u), 0.0f};
   const float hi = float(x);
   if (!(fabsf(hi) < INFINITY)) return {hi, 0.0f};  // beyond the float range
   return {hi, float(x - double(hi))};
+}
+NW_HD dd dd_from_double(double x) {
+  const uint64_t b = d2u(x);
+  const uint32_t hw = uint32_t(b >> 32), lw = uint32_t(b);
+  if (dd_split_range(hw) < kDdSplit) return dd_split_bits(hw, lw);
+  return dd_from_double_slow(x);
+}
+NW_HD dd dd_from_double_near(double x) {
+  const uint64_t b = d2u(x);
+  const uint32_t hw = uint32_t(b >> 32), lw = uint32_t(b);
+  if (dd_split_range(hw) < kDdSplit) return dd_split_near(hw, lw);
+  return dd_from_double_slow(x);
+}
+// for values that are often exactly zero (components of the area and edge
+// vectors of an axis-aligned mesh): zero does not leave the fast path
+NW_HD dd dd_from_double_z(double x) {
+  const uint64_t b = d2u(x);
+  const uint32_t hw = uint32_t(b >> 32), lw = uint32_t(b);
+  const bool zero = (hw * 2u | lw) == 0;
+  if (dd_split_range(hw) < kDdSplit || zero) {
+    const dd r = dd_split_bits(hw, lw);
+    return {zero ? 0.0f : r.hi, zero ? 0.0f : r.lo};
+  }
+  return dd_from_double_slow(x);
+}
+// three splits with one range test
+NW_HD void dd_from_double3(const double x[3], dd o[3]) {
+  const uint64_t b0 = d2u(x[0]), b1 = d2u(x[1]), b2 = d2u(x[2]);
+  const uint32_t h0 = uint32_t(b0 >> 32), h1 = uint32_t(b1 >> 32), h2 = uint32_t(b2 >> 32);
+  const uint32_t r0 = dd_split_range(h0), r1 = dd_split_range(h1), r2 = dd_split_range(h2);
+  const uint32_t m = r0 > r1 ? r0 : r1;
+  if ((m > r2 ? m : r2) < kDdSplit) {
+    o[0] = dd_split_bits(h0, uint32_t(b0));
+    o[1] = dd_split_bits(h1, uint32_t(b1));
+    o[2] = dd_split_bits(h2, uint32_t(b2));
+  } else {
+    o[0] = r0 < kDdSplit ? dd_split_bits(h0, uint32_t(b0)) : dd_from_double_slow(x[0]);
+    o[1] = r1 < kDdSplit ? dd_split_bits(h1, uint32_t(b1)) : dd_from_double_slow(x[1]);
+    o[2] = r2 < kDdSplit ? dd_split_bits(h2, uint32_t(b2)) : dd_from_double_slow(x[2]);
+  }
 }
 
 NW_HD dd operator-(dd a) { return {-a.hi, -a.lo}; }
@@ -275,19 +343,23 @@ NW_HD dd dd_dot3(dd a0, dd b0, dd a1, dd b1, dd a2, dd b2) {
   return fast_two_sum(s.hi, err);
 }
 
-// 1/x: float seed refined by one Newton step in double-word arithmetic.
-// x == 0 gives inf (as the FP64 reciprocal does); non-finite x its float
-// reciprocal.
+// 1/x: float seed r0 (within 2^-22), e = 1 - x r0 with the product kept to
+// 48 bits, r0 (1 + e + e^2) in double-word arithmetic. x == 0 gives inf (as
+// the FP64 reciprocal does); non-finite x its float reciprocal.
 NW_HD dd dd_rcp(dd x) {
-  x = fast_two_sum(x.hi, x.lo);  // |lo| <= ulp(hi)/2 keeps the seed within 2^-23
+  x = fast_two_sum(x.hi, x.lo);  // |lo| <= ulp(hi)/2 keeps the seed's error from the head alone
+#ifdef __CUDA_ARCH__
+  float r0;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r0) : "f"(x.hi));
+#else
   const float r0 = 1.0f / x.hi;
+#endif
   if (x.hi == 0.0f || !(fabsf(r0) < INFINITY)) return {r0, 0.0f};
-  // e = 1 - x r0 with the product kept to 48 bits
   const float p = fmul(x.hi, r0);
   float pe = ffma(x.hi, r0, -p);
   pe = ffma(x.lo, r0, pe);
   const float e = fsub(fsub(1.0f, p), pe);
-  return fast_two_sum(r0, fmul(r0, e));
+  return fast_two_sum(r0, fmul(r0, ffma(e, e, e)));
 }
 
 NW_HD dd dd_abs(dd a) { return a.hi < 0.0f ? -a : a; }

@@ -640,7 +640,7 @@ nw_status nw_assemble_momentum_edges(nw_linsys* ls, const nw_momentum_fields* f,
       NW_CUDA(cudaGetLastError());
       ls->pristine = false;
     } else {
-      launch_momentum_edges(ls->stream, E, 0, E, ls->edges.p, *f, *o, ls->buf.p);
+      launch_momentum_edges(ls->stream, 0, E, ls->edges.p, *f, *o, ls->buf.p);
       momentum_rows(ls, o->relax);
     }
     end_timing(ls);
@@ -655,7 +655,7 @@ nw_status nw_assemble_momentum_edge_range(nw_linsys* ls, const nw_momentum_field
     const int64_t E = ls->g.num_edges;
     if (edge_begin < 0 || edge_end > E || edge_begin > edge_end)
       fail(NW_INVALID_ARG, "edge range out of bounds");
-    launch_momentum_edges(ls->stream, E, edge_begin, edge_end, ls->edges.p, *f, *o, ls->buf.p);
+    launch_momentum_edges(ls->stream, edge_begin, edge_end, ls->edges.p, *f, *o, ls->buf.p);
     NW_CUDA(cudaGetLastError());
   });
 }

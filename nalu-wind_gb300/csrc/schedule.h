@@ -19,7 +19,7 @@
 namespace nw {
 
 constexpr int kFusedChunk = 256;  // edges per edge chunk (one per thread)
-constexpr int kFusedBlock = 85;   // node rows per row block (3 threads each)
+constexpr int kFusedBlock = 80;   // node rows per row block (ten per warp)
 
 struct FusedSchedule {
   int64_t chunks = 0;       // edge chunks
