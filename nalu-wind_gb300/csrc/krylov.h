@@ -63,8 +63,9 @@ class KrylovSolver {
   void setup(const DevCsr& A, int m, cudaStream_t s);
   // Colour classes of the multicolour Gauss-Seidel sweep (rows of class 0,
   // then class 1, ...; cptr on the host): builds the class-ordered sliced
-  // copy of the off-diagonal entries the sweep reads.
-  void setup_colors(const std::vector<int32_t>& rows, const std::vector<int64_t>& cptr,
+  // copy of the off-diagonal entries the sweep reads. dof: rows per node,
+  // class (colour, d) holding row d of the colour's nodes.
+  void setup_colors(const std::vector<int32_t>& rows, const std::vector<int64_t>& cptr, int dof,
                     cudaStream_t s);
   // Recompute diagonal-dependent data after the values changed.
   void refresh(cudaStream_t s);
@@ -163,6 +164,9 @@ class KrylovSolver {
   // columns, CSR positions (for the value gathers) and values.
   std::vector<int64_t> gs_cptr_, gs_slice0_;  // host: class row / slice starts
   DeviceArray<int32_t> gs_rows_, gs_len_, gs_cols_, gs_map_;
+  DeviceArray<int32_t> gs_own_;  // first entry of the row's own node (gs_dof_ > 1)
+  std::vector<int64_t> gs_size_; // per colour: entries of one dof class
+  int gs_dof_ = 1;               // > 1: a colour's dof classes are swept by one kernel
   DeviceArray<int64_t> gs_off_;
   DeviceArray<double> gs_vals_;
   DeviceArray<float> gs_vals32_;

@@ -443,7 +443,7 @@ nw_status nw_linsys_finalize(nw_linsys* ls) {
     A.row_ptr_host = g.row_ptr.data();
     A.col_idx_host = g.col_idx.data();
     ls->solver.setup(A, std::max(ls->cfg.kspace, ls->cfg.inner_kspace), s);
-    ls->solver.setup_colors(ls->color_rows_host, ls->color_ptr, s);
+    ls->solver.setup_colors(ls->color_rows_host, ls->color_ptr, ls->num_dof, s);
     NW_CUDA(cudaStreamSynchronize(s));
     ls->finalized = true;
   });
@@ -1020,7 +1020,7 @@ nw_status nw_linsys_checkpoint_load(nw_linsys* ls, const char* path, double* x, 
       A.row_ptr_host = g.row_ptr.data();
       A.col_idx_host = g.col_idx.data();
       ls->solver.setup(A, std::max(ls->cfg.kspace, ls->cfg.inner_kspace), ls->stream);
-      ls->solver.setup_colors(ls->color_rows_host, ls->color_ptr, ls->stream);
+      ls->solver.setup_colors(ls->color_rows_host, ls->color_ptr, ls->num_dof, ls->stream);
     }
     ls->history = hist;
     ls->last_report = h.report;
