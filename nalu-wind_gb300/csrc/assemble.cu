@@ -312,7 +312,7 @@ __global__ void __launch_bounds__(kThreads)
 __device__ __forceinline__ dd van_leer_dd(dd dqm, dd dqp, dd eps) {
   const dd p = dqm * dqp;
   const dd s = dqm + dqp;
-  return scale2(p + dd_abs(p), 2.0f) * dd_rcp(s * s + eps);
+  return scale2(p + dd_abs(p), 2.0f) * dd_rcp_fast(s * s + eps);
 }
 
 // ---------------------------------------------------------------------------
@@ -393,7 +393,7 @@ __device__ __forceinline__ void momentum_edge(int64_t e, const MomentumIn& in, c
   const dd mdot = dd_from_double_near(in.mdot[e]), pec = ldd(in.pec + e);
   const bool up = dd_gt0(mdot);
   const dd asq = dd_dot3(av[0], av[0], av[1], av[1], av[2], av[2]);
-  const dd hinv = dd_rcp(dd_dot3(av[0], hdx[0], av[1], hdx[1], av[2], hdx[2]));  // 2 / (A.dx)
+  const dd hinv = dd_rcp_fast(dd_dot3(av[0], hdx[0], av[1], hdx[1], av[2], hdx[2]));  // 2 / (A.dx)
   const dd inv_axdx = scale2(hinv, 0.5f);
   const dd mp = mdot * pec;
   // g: the sum (not the mean) of the two nodal gradients; corr: the factor of

@@ -10,7 +10,7 @@
 //   add:  |err| <= 2 u^2 (|a| + |b|)      (relative to the operand sizes,
 //                                          not to the possibly cancelling sum)
 //   mul:  |err| <= 4 u^2 |a b|
-//   rcp:  |err| <= 3 u^2 / |x|            (a quadratic step from a float seed)
+//   rcp:  |err| <= 3 u^2 / |x|            (one step from a float seed)
 // Conversions from double keep the top 48 significand bits (the split error
 // is <= 2^-48 relative); dd -> double rounds hi + lo once. The
 // exponent range is the float range: |x| >= 2^128 becomes infinite, and
@@ -343,11 +343,25 @@ NW_HD dd dd_dot3(dd a0, dd b0, dd a1, dd b1, dd a2, dd b2) {
   return fast_two_sum(s.hi, err);
 }
 
-// 1/x: float seed r0 (within 2^-22), e = 1 - x r0 with the product kept to
-// 48 bits, r0 (1 + e + e^2) in double-word arithmetic. x == 0 gives inf (as
-// the FP64 reciprocal does); non-finite x its float reciprocal.
+// 1/x: float seed refined by one Newton step in double-word arithmetic.
+// x == 0 gives inf (as the FP64 reciprocal does); non-finite x its float
+// reciprocal.
 NW_HD dd dd_rcp(dd x) {
-  x = fast_two_sum(x.hi, x.lo);  // |lo| <= ulp(hi)/2 keeps the seed's error from the head alone
+  x = fast_two_sum(x.hi, x.lo);  // |lo| <= ulp(hi)/2 keeps the seed within 2^-23
+  const float r0 = 1.0f / x.hi;
+  if (x.hi == 0.0f || !(fabsf(r0) < INFINITY)) return {r0, 0.0f};
+  // e = 1 - x r0 with the product kept to 48 bits
+  const float p = fmul(x.hi, r0);
+  float pe = ffma(x.hi, r0, -p);
+  pe = ffma(x.lo, r0, pe);
+  const float e = fsub(fsub(1.0f, p), pe);
+  return fast_two_sum(r0, fmul(r0, e));
+}
+// The same from the approximate float reciprocal (within 2^-22, a third of
+// the division's instructions) with a quadratic step r0 (1 + e + e^2), which
+// leaves the same error bound.
+NW_HD dd dd_rcp_fast(dd x) {
+  x = fast_two_sum(x.hi, x.lo);
 #ifdef __CUDA_ARCH__
   float r0;
   asm("rcp.approx.f32 %0, %1;" : "=f"(r0) : "f"(x.hi));

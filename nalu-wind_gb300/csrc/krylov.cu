@@ -692,7 +692,7 @@ constexpr int kMaxDof = 3;
 constexpr int kGsNodeBatch = 20, kGsNodeBlock = 64;
 struct GsNodeArgs {
   int64_t cnt;
-  const int32_t *rows, *len, *own;  // of class (colour, 0)
+  const int32_t *rows, *len, *own;  // of class (colour, 0); own of the first colour
   const int64_t* off;
   int64_t size;  // entries of one dof class (the dof classes follow each other)
   int dof, nseq, nfwd, fresh, first;
@@ -1491,7 +1491,7 @@ void KrylovSolver::sgs(const VT* vals, const T* rd, const T* x, T* y, cudaStream
       const int64_t b = gs_cptr_[c * dof];
       g.rows = gs_rows_.p + b;
       g.len = gs_len_.p + b;
-      g.own = gs_own_.p + b;
+      g.own = gs_own_.p;
       g.off = gs_off_.p + gs_slice0_[c * dof];
       g.size = gs_size_[c];
       if (forward)
@@ -1599,11 +1599,11 @@ void KrylovSolver::setup_colors(const std::vector<int32_t>& rows,
         nodes = rows[b0 + k] % dof == 0 && rows[cptr[c] + k] == rows[b0 + k] + c % dof && len[cptr[c] + k] == len[b0 + k];
     }
     if (nodes) {
-      std::vector<int32_t> own(n, 0);
-      for (int64_t k = 0; k < n; ++k) {
-        const int32_t i = rows[k], node = i - i % dof;
+      std::vector<int32_t> own(cptr[1]);  // only the first colour's is used
+      for (int64_t k = 0; k < cptr[1]; ++k) {
+        const int32_t i = rows[k];
         int32_t q = 0;
-        for (int64_t p = A_.row_ptr_host[i]; p < A_.row_ptr_host[i + 1] && A_.col_idx_host[p] < node; ++p) ++q;
+        for (int64_t p = A_.row_ptr_host[i]; p < A_.row_ptr_host[i + 1] && A_.col_idx_host[p] < i; ++p) ++q;
         own[k] = q;
       }
       gs_own_.upload(own, s);

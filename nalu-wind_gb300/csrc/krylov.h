@@ -164,7 +164,7 @@ class KrylovSolver {
   // columns, CSR positions (for the value gathers) and values.
   std::vector<int64_t> gs_cptr_, gs_slice0_;  // host: class row / slice starts
   DeviceArray<int32_t> gs_rows_, gs_len_, gs_cols_, gs_map_;
-  DeviceArray<int32_t> gs_own_;  // first entry of the row's own node (gs_dof_ > 1)
+  DeviceArray<int32_t> gs_own_;  // first entry of the own node, first colour (gs_dof_ > 1)
   std::vector<int64_t> gs_size_; // per colour: entries of one dof class
   int gs_dof_ = 1;               // > 1: a colour's dof classes are swept by one kernel
   DeviceArray<int64_t> gs_off_;
