@@ -12,17 +12,18 @@ using ScalarOpts = nw_scalar_opts;
 using ContinuityOpts = nw_continuity_opts;
 using MomentumOpts = nw_momentum_opts;
 
-// 8-byte coefficient slots per edge written by the edge phase: scalar, six
-// FP64 SoA arrays of E; continuity, one 16-byte record (f, tmdot as float
+// 8-byte coefficient slots per edge written by the edge phase: scalar, one
+// 32-byte record (a01, a10, flux in FP64); continuity, one 16-byte record (f, tmdot as float
 // pairs) per edge; momentum, one 96-byte record per edge (nine FP64 CSR
 // entries and three float pairs, see momentum_edge).
-constexpr int kScalarCoefs = 6;
+constexpr int kScalarCoefs = 4;
 constexpr int kContinuityCoefs = 2;
 constexpr int kMomentumCoefs = 12;
 
-void launch_scalar_edges(cudaStream_t s, int64_t E, const int2* edges,
+// nodebuf: N doubles of scratch
+void launch_scalar_edges(cudaStream_t s, int64_t E, int64_t N, const int2* edges,
                          const nw_scalar_fields& f, const ScalarOpts& o,
-                         double* buf);
+                         double* buf, double* nodebuf);
 void launch_continuity_edges(cudaStream_t s, int64_t E, const int2* edges,
                              const nw_continuity_fields& f,
                              const ContinuityOpts& o, double* buf);

@@ -503,7 +503,7 @@ nw_status nw_assemble_scalar_edges(nw_linsys* ls, const nw_scalar_fields* f,
     if (!(o->relax != 0.0)) fail(NW_INVALID_ARG, "relaxation factor is zero");
     begin_timing(ls);
     const int64_t E = ls->g.num_edges;
-    launch_scalar_edges(ls->stream, E, ls->edges.p, *f, *o, ls->buf.p);
+    launch_scalar_edges(ls->stream, E, ls->g.num_nodes, ls->edges.p, *f, *o, ls->buf.p, ls->nodebuf.p);
     launch_rows(ls->stream, 0, ls->g.node_rows, ls->inc_ptr.p, ls->inc.p,
                 ls->diag_pos.p, ls->row_ptr.p, ls->buf.p, E, o->relax,
                 ls->values.p, ls->rhs.p, write_mode(ls), ls->stage_bytes[0]);
