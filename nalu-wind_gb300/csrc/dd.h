@@ -263,6 +263,16 @@ NW_HD dd dd_from_double_z(double x) {
   }
   return dd_from_double_slow(x);
 }
+NW_HD dd dd_from_double_near_z(double x) {
+  const uint64_t b = d2u(x);
+  const uint32_t hw = uint32_t(b >> 32), lw = uint32_t(b);
+  const bool zero = (hw * 2u | lw) == 0;
+  if (dd_split_range(hw) < kDdSplit || zero) {
+    const dd r = dd_split_near(hw, lw);
+    return {zero ? 0.0f : r.hi, zero ? 0.0f : r.lo};
+  }
+  return dd_from_double_slow(x);
+}
 // three splits with one range test
 NW_HD void dd_from_double3(const double x[3], dd o[3]) {
   const uint64_t b0 = d2u(x[0]), b1 = d2u(x[1]), b2 = d2u(x[2]);
