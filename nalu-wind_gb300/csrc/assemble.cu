@@ -220,6 +220,13 @@ __global__ void __launch_bounds__(kThreads)
 // w = |A|^2 / (A.dx), k = A - w dx, then tmdot /= tau. This is the
 // reference expression regrouped; the parity tests bound the difference by
 // eps times the running magnitude of each entry.
+//
+// The edge phase is bound by its 580 instructions an edge (56 % of the issue
+// slots) and the latency of two random records: 88 us on 128x128x64 hexes with
+// 16-byte record loads and 4 resident blocks a SM. Records read as 32-byte
+// loads and summed on arrival leave 40 registers and six blocks: the whole
+// assembly takes 147 us, 159 before (4 blocks 158, 5 blocks 150). PLAIN: the
+// default noc = 1 needs no product with it.
 constexpr int kNodeStride = 8;  // dd slots (8 bytes each) per node
 
 __device__ __forceinline__ dd ldd(const double* p) { return dd_from_double(*p); }
@@ -248,7 +255,8 @@ __global__ void __launch_bounds__(kThreads)
       ldd(Gpdx + 3 * n + 2) * iu, ldd(pressure + n));
 }
 
-__global__ void __launch_bounds__(kThreads)
+template <bool PLAIN>
+__global__ void __launch_bounds__(kThreads, 6)
     continuity_edge_fast_k(int64_t E, const int2* __restrict__ edges,
                            const double* __restrict__ coords,
                            const dd* __restrict__ nodebuf,
@@ -259,42 +267,46 @@ __global__ void __launch_bounds__(kThreads)
   if (e >= E) return;
   const int2 lr = edges[e];
   const int64_t L = lr.x, R = lr.y;
-  dd nl[8], nr[8];
+  // sums over the two nodes; a record is two 32-byte loads (four 16-byte
+  // loads cost twice the L1 lookups)
+  dd n[7];
   {
-    const float4* pl = reinterpret_cast<const float4*>(nodebuf + kNodeStride * L);
-    const float4* pr = reinterpret_cast<const float4*>(nodebuf + kNodeStride * R);
+    double a[4], b[4];
+    const double* pl = reinterpret_cast<const double*>(nodebuf + kNodeStride * L);
+    const double* pr = reinterpret_cast<const double*>(nodebuf + kNodeStride * R);
+    auto pair = [](double x) { return dd{__int_as_float(__double2loint(x)), __int_as_float(__double2hiint(x))}; };
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const float4 a = pl[k], b = pr[k];
-      nl[2 * k] = {a.x, a.y};
-      nl[2 * k + 1] = {a.z, a.w};
-      nr[2 * k] = {b.x, b.y};
-      nr[2 * k + 1] = {b.z, b.w};
+    for (int h = 0; h < 2; ++h) {
+      ld32<true>(pl + 4 * h, a);
+      ld32<true>(pr + 4 * h, b);
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (4 * h + k < 7) n[4 * h + k] = pair(a[k]) + pair(b[k]);
     }
   }
   dd av[3], dx[3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
-    av[d] = ldd(area + 3 * e + d);
-    dx[d] = dd_from_double(coords[3 * R + d] - coords[3 * L + d]);
+    av[d] = dd_from_double_z(area[3 * e + d]);
+    dx[d] = dd_from_double_z(coords[3 * R + d] - coords[3 * L + d]);
   }
   const dd asq = dd_dot3(av[0], av[0], av[1], av[1], av[2], av[2]);
   const dd axdx = dd_dot3(av[0], dx[0], av[1], dx[1], av[2], dx[2]);
   const dd w = asq * dd_rcp(axdx);
-  const dd projTimeScale = scale2(nl[0] + nr[0], 0.5f);
-  dd mg[3], g[3], c[3];
+  const dd projTimeScale = scale2(n[0], 0.5f);
+  dd mg[3], c[3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
-    g[d] = nl[4 + d] + nr[4 + d];
-    mg[d] = (nl[1 + d] + nr[1 + d]) + g[d];
+    mg[d] = n[1 + d] + n[4 + d];
     c[d] = av[d] - w * dx[d];
   }
   // sum (rho u + G p / A_p) . A and the non-orthogonal correction
   // sum (A - w dx) . (G p / A_p), as three-term dots
   const dd flux = dd_dot3(mg[0], av[0], mg[1], av[1], mg[2], av[2]);
-  const dd corr = dd_dot3(c[0], g[0], c[1], g[1], c[2], g[2]);
+  dd corr = dd_dot3(c[0], n[4], c[1], n[5], c[2], n[6]);
+  if (!PLAIN) corr = noc * corr;
   dd tmdot = -(projTimeScale * dd_from_double(pressure[R] - pressure[L]) * w);
-  tmdot = (tmdot + scale2(flux - noc * corr, 0.5f)) * inv_tau;
+  tmdot = (tmdot + scale2(flux - corr, 0.5f)) * inv_tau;
   const dd f = -(w * projTimeScale * inv_tau);
   reinterpret_cast<float4*>(buf)[e] = make_float4(f.hi, f.lo, tmdot.hi, tmdot.lo);
 }
@@ -1057,9 +1069,16 @@ void launch_continuity_edge_range(cudaStream_t s, int64_t n0, int64_t n1, int64_
     if (n1 > n0)
       continuity_node_k<<<grid_for(n1 - n0), kThreads, 0, s>>>(
           n0, n1, f.velocity, f.dpdx, f.density, f.pressure, f.udiag, nb);
-    if (n)
-      continuity_edge_fast_k<<<grid_for(n), kThreads, 0, s>>>(
-          n, er, f.coords, nb, f.pressure, ar, dd_param(o.noc_fac), dd_param(1.0 / o.tau_scale), b);
+    if (n) {
+      auto go = [&](auto kernel) {
+        kernel<<<grid_for(n), kThreads, 0, s>>>(n, er, f.coords, nb, f.pressure, ar, dd_param(o.noc_fac),
+                                                dd_param(1.0 / o.tau_scale), b);
+      };
+      if (o.noc_fac == 1.0)
+        go(continuity_edge_fast_k<true>);
+      else
+        go(continuity_edge_fast_k<false>);
+    }
   } else if (n) {
     ContinuityDD c;
     c.noc = dd_param(o.noc_fac);

@@ -1,7 +1,7 @@
 """The input producers' forms: the mass flow for each pair of non-orthogonal
 and interpolation factors (the default pair has its own kernel) and the nodal
-gradients on rows of one to many edges, against the formulas in NumPy FP64. Tolerance 1e-12 of the summed magnitudes, as for every
-kernel in float pairs."""
+gradients on rows of one to many edges, against the formulas in NumPy FP64.
+Tolerance 1e-12 of the summed magnitudes, as for every kernel in float pairs."""
 import numpy as np
 import pytest
 
