@@ -477,18 +477,114 @@ __global__ void __launch_bounds__(kBlock, kMdot4PerSm)
   }
 }
 
+// ---------------------------------------------------------------------------
+// GMRES least squares on the device. A warp applies the previous Givens
+// rotations to the new Hessenberg column, one thread forms the next rotation,
+// updates the rotated rhs g and the residual estimate, and records
+// convergence; the host reads the control words one chunk of iterations
+// behind instead of waiting for every column. Every operation is an
+// explicitly rounded FP64 add, multiply, divide or square root (no fused
+// multiply-adds), the same arithmetic as the host restatement of the
+// solver, so iterates and histories do not depend on where it runs.
+__global__ void givens_init_k(GivensDev G, double g0) {
+  if (threadIdx.x != 0) return;
+  for (int k = 0; k <= G.m; ++k) G.g[k] = 0.0;
+  G.g[0] = g0;
+  G.ctl[kCtlDone] = 0;
+  G.ctl[kCtlIts] = 0;
+  G.ctl[kCtlStatus] = NW_OK;
+  G.ctl[kCtlBasis] = 0;
+}
+
+// The previous rotations applied to column j, by one warp: the last entry,
+// which the column's own rotation takes, is left in H(j, j). They need the
+// coefficients only, so an extra block of the multi-axpy that forms the new
+// vector and its norm runs them meanwhile. The rotations are a serial chain
+// a <- c_k h_{k+1} - s_k a; the products with h and the entries of the column
+// are formed by 32 lanes at a time, so a rotation costs one multiply and one
+// add of latency (0.14 us) instead of a load of the previous store and six
+// operations (0.5 us).
+__device__ __noinline__ void givens_rotate(const GivensDev& G, int j, const double* __restrict__ hs) {
+  const int lane = threadIdx.x & 31;
+  if (G.ctl[kCtlDone]) return;
+  const int m = G.m;
+  double* H = G.H;
+  double a = hs[0];
+  for (int k0 = 0; k0 < j; k0 += 32) {
+    const int k = k0 + lane;
+    const bool on = k < j;
+    const double cs = on ? G.cs[k] : 0.0, sn = on ? G.sn[k] : 0.0, h = on ? hs[k + 1] : 0.0;
+    const double p = __dmul_rn(sn, h), q = __dmul_rn(cs, h);
+    double ak = 0.0;
+    const int cnt = min(32, j - k0);
+    for (int l = 0; l < cnt; ++l) {
+      const double snl = __shfl_sync(0xffffffffu, sn, l), ql = __shfl_sync(0xffffffffu, q, l);
+      if (lane == l) ak = a;
+      a = __dadd_rn(__dmul_rn(-snl, a), ql);
+    }
+    if (on) H[size_t(k) * m + j] = __dadd_rn(__dmul_rn(cs, ak), p);
+  }
+  if (lane == 0) H[size_t(j) * m + j] = a;
+}
+
+// The rotation of column j itself, from the norm of the new vector: one
+// thread, beside the scaling of that vector.
+__device__ void givens_finish(const GivensCol& c) {
+  const GivensDev& G = c.G;
+  if (G.ctl[kCtlDone]) return;
+  const int m = G.m, j = c.j;
+  double* H = G.H;
+  const double hn = c.hn[0], a = H[size_t(j) * m + j];
+  const double bb = hn;
+  const double den = __dsqrt_rn(__dadd_rn(__dmul_rn(a, a), __dmul_rn(bb, bb)));
+  H[size_t(j + 1) * m + j] = bb;
+  if (!(den > 0.0) || !isfinite(den)) {
+    G.ctl[kCtlStatus] = isfinite(den) ? NW_BREAKDOWN : NW_NAN_DETECTED;
+    G.ctl[kCtlBasis] = j;
+    G.ctl[kCtlDone] = 1;
+    return;
+  }
+  const double cj = __ddiv_rn(a, den), sj = __ddiv_rn(bb, den);
+  G.cs[j] = cj;
+  G.sn[j] = sj;
+  H[size_t(j) * m + j] = den;
+  H[size_t(j + 1) * m + j] = 0.0;
+  const double gj = G.g[j], gn = __dmul_rn(-sj, gj);
+  G.g[j + 1] = gn;
+  G.g[j] = __dmul_rn(cj, gj);
+  G.ctl[kCtlIts] = j + 1;
+  const double rel = __ddiv_rn(fabs(gn), c.div);
+  G.hist[j] = __ddiv_rn(__dmul_rn(rel, c.hist_mul), c.hist_div);
+  if (!isfinite(rel)) {
+    G.ctl[kCtlStatus] = NW_NAN_DETECTED;
+    G.ctl[kCtlBasis] = j + 1;
+    G.ctl[kCtlDone] = 1;
+  } else if (rel <= c.tol || hn == 0.0) {
+    G.ctl[kCtlBasis] = j + 1;
+    G.ctl[kCtlDone] = 1;
+  }
+}
+
 // w -= V h for groups of four elements, and the norm of the updated w
 // (elements below n only): per-block partial sums of |w|^2, their sum and its
-// root in the last block.
+// root in the last block. Block 0 applies the earlier Givens rotations to the
+// new Hessenberg column meanwhile: in the scaling kernel, which had the whole
+// column, that chain took 3 of the kernel's 5.4 us at 0.32 M rows.
 __global__ void __launch_bounds__(kBlock)
     maxpy4_k(int64_t n, int nv, const float* __restrict__ V, int64_t ld,
              const double* __restrict__ h, float* __restrict__ w,
-             double* __restrict__ nrm_partial, double* __restrict__ nrm, int* __restrict__ ticket) {
+             double* __restrict__ nrm_partial, double* __restrict__ nrm, int* __restrict__ ticket,
+             GivensDev G, int j) {
+  if (blockIdx.x == 0) {
+    if (threadIdx.x < 32) givens_rotate(G, j, h);
+    return;
+  }
+  const unsigned block = blockIdx.x - 1;
   __shared__ float hs[1024];
   __shared__ double red[kBlock / 32], sh[kBlock];
   for (int k = threadIdx.x; k < nv; k += blockDim.x) hs[k] = float(h[k]);
   __syncthreads();
-  const int64_t g = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int64_t g = int64_t(block) * blockDim.x + threadIdx.x;
   const int64_t ng = (n + 3) >> 2;
   float ss = 0.f, cc = 0.f;
   if (g < ng) {
@@ -528,16 +624,17 @@ __global__ void __launch_bounds__(kBlock)
   if (threadIdx.x == 0) {
     double t = 0.0;
     for (int q = 0; q < kBlock / 32; ++q) t += red[q];
-    nrm_partial[blockIdx.x] = t;
+    nrm_partial[block] = t;
   }
-  if (!last_block(ticket, gridDim.x)) return;
-  const double t = block_tree_sum(gridDim.x, nrm_partial, sh);
+  if (!last_block(ticket, gridDim.x - 1)) return;
+  const double t = block_tree_sum(gridDim.x - 1, nrm_partial, sh);
   if (threadIdx.x == 0) nrm[0] = sqrt(t);
 }
 
 // FP64 w -= sum_k h[k] V[k] (h on the device); with nrm, also ||w|| of the
 // result: partial sums per 256 elements (one per thread, warp trees, warps in
-// order), their sum and its root in the last block.
+// order), their sum and its root in the last block. With gd, block 0 applies
+// the earlier Givens rotations to column j (coefficients hcol) meanwhile.
 //
 // EPT elements a thread, 256 apart, so that a thread keeps EPT independent
 // fma chains and loads in flight and the warp trees of EPT partial sums run
@@ -551,12 +648,18 @@ template <int EPT>
 __global__ void __launch_bounds__(kBlock)
     maxpy64_k(int64_t n, int nv, const double* __restrict__ V, int64_t ld, const double* __restrict__ h,
               double* __restrict__ w, double* __restrict__ nrm_partial, double* __restrict__ nrm,
-              int* __restrict__ ticket) {
+              int* __restrict__ ticket, GivensDev gd, int j, const double* __restrict__ hcol) {
+  const unsigned rot = gd.H ? 1 : 0;
+  if (rot && blockIdx.x == 0) {
+    if (threadIdx.x < 32) givens_rotate(gd, j, hcol);
+    return;
+  }
+  const unsigned block = blockIdx.x - rot;
   __shared__ double hs[kMaxVecs];
   __shared__ double red[EPT][kBlock / 32], sh[kBlock];
   for (int k = threadIdx.x; k < nv; k += kBlock) hs[k] = h[k];
   __syncthreads();
-  const int64_t i0 = int64_t(blockIdx.x) * (EPT * kBlock) + threadIdx.x;
+  const int64_t i0 = int64_t(block) * (EPT * kBlock) + threadIdx.x;
   double acc[EPT];
   if (i0 + (EPT - 1) * kBlock < n) {
 #pragma unroll
@@ -599,13 +702,13 @@ __global__ void __launch_bounds__(kBlock)
   if (lane % (32 / EPT) == 0) red[lane / (32 / EPT)][threadIdx.x >> 5] = acc[0];
   __syncthreads();
   const int G = int((n + kBlock - 1) / kBlock);
-  if (threadIdx.x < EPT && int(blockIdx.x) * EPT + int(threadIdx.x) < G) {
+  if (threadIdx.x < EPT && int(block) * EPT + int(threadIdx.x) < G) {
     double t = red[threadIdx.x][0];
 #pragma unroll
     for (int q = 1; q < kBlock / 32; ++q) t += red[threadIdx.x][q];
-    nrm_partial[blockIdx.x * EPT + threadIdx.x] = t;
+    nrm_partial[block * EPT + threadIdx.x] = t;
   }
-  if (!last_block(ticket, gridDim.x)) return;
+  if (!last_block(ticket, gridDim.x - rot)) return;
   const double t = block_tree_sum(G, nrm_partial, sh);
   if (threadIdx.x == 0) nrm[0] = sqrt(t);
 }
@@ -999,110 +1102,15 @@ __global__ void __launch_bounds__(kBlock)
   }
 }
 
-// ---------------------------------------------------------------------------
-// GMRES least squares on the device. One thread applies the previous
-// Givens rotations to the new Hessenberg column, forms the next rotation,
-// updates the rotated rhs g and the residual estimate, and records
-// convergence; the host reads the control words one chunk of iterations
-// behind instead of waiting for every column. Every operation is an
-// explicitly rounded FP64 add, multiply, divide or square root (no fused
-// multiply-adds), the same arithmetic as the host restatement of the
-// solver, so iterates and histories do not depend on where it runs.
-struct GivensDev {
-  double *H, *cs, *sn, *g, *hist;
-  int* ctl;  // done, iterations of the cycle, status, basis vectors
-  int m;
-};
-enum { kCtlDone = 0, kCtlIts = 1, kCtlStatus = 2, kCtlBasis = 3 };
-
-__global__ void givens_init_k(GivensDev G, double g0) {
-  if (threadIdx.x != 0) return;
-  for (int k = 0; k <= G.m; ++k) G.g[k] = 0.0;
-  G.g[0] = g0;
-  G.ctl[kCtlDone] = 0;
-  G.ctl[kCtlIts] = 0;
-  G.ctl[kCtlStatus] = NW_OK;
-  G.ctl[kCtlBasis] = 0;
-}
-
-// Column j: h = hs[0..j], hn = ||w||. rel = |g[j+1]| / div; the history
-// entry is rel * hist_mul / hist_div; the cycle stops when rel <= tol or
-// hn == 0 (basis j + 1), on a non-finite estimate (basis j + 1) or when the
-// rotation breaks down (basis j).
-struct GivensCol {
-  GivensDev G;
-  int j;
-  const double *hs, *hn;
-  double tol, div, hist_mul, hist_div;
-};
-
-// By one warp. The rotations are a serial chain a <- c_k h_{k+1} - s_k a; the
-// products with h and the entries of the column are formed by 32 lanes at a
-// time, so a rotation costs one multiply and one add of latency (0.14 us)
-// instead of a load of the previous store and six operations (0.5 us).
-__device__ void givens_step(const GivensCol& c) {
-  const GivensDev& G = c.G;
-  const int lane = threadIdx.x & 31;
-  if (G.ctl[kCtlDone]) return;
-  const int m = G.m, j = c.j;
-  double* H = G.H;
-  const double hn = c.hn[0];
-  double a = c.hs[0];
-  for (int k0 = 0; k0 < j; k0 += 32) {
-    const int k = k0 + lane;
-    const bool on = k < j;
-    const double cs = on ? G.cs[k] : 0.0, sn = on ? G.sn[k] : 0.0, h = on ? c.hs[k + 1] : 0.0;
-    const double p = __dmul_rn(sn, h), q = __dmul_rn(cs, h);
-    double ak = 0.0;
-    const int cnt = min(32, j - k0);
-    for (int l = 0; l < cnt; ++l) {
-      const double snl = __shfl_sync(0xffffffffu, sn, l), ql = __shfl_sync(0xffffffffu, q, l);
-      if (lane == l) ak = a;
-      a = __dadd_rn(__dmul_rn(-snl, a), ql);
-    }
-    if (on) H[size_t(k) * m + j] = __dadd_rn(__dmul_rn(cs, ak), p);
-  }
-  if (lane != 0) return;
-  const double bb = hn;
-  const double den = __dsqrt_rn(__dadd_rn(__dmul_rn(a, a), __dmul_rn(bb, bb)));
-  H[size_t(j) * m + j] = a;
-  H[size_t(j + 1) * m + j] = bb;
-  if (!(den > 0.0) || !isfinite(den)) {
-    G.ctl[kCtlStatus] = isfinite(den) ? NW_BREAKDOWN : NW_NAN_DETECTED;
-    G.ctl[kCtlBasis] = j;
-    G.ctl[kCtlDone] = 1;
-    return;
-  }
-  const double cj = __ddiv_rn(a, den), sj = __ddiv_rn(bb, den);
-  G.cs[j] = cj;
-  G.sn[j] = sj;
-  H[size_t(j) * m + j] = den;
-  H[size_t(j + 1) * m + j] = 0.0;
-  const double gj = G.g[j], gn = __dmul_rn(-sj, gj);
-  G.g[j + 1] = gn;
-  G.g[j] = __dmul_rn(cj, gj);
-  G.ctl[kCtlIts] = j + 1;
-  const double rel = __ddiv_rn(fabs(gn), c.div);
-  G.hist[j] = __ddiv_rn(__dmul_rn(rel, c.hist_mul), c.hist_div);
-  if (!isfinite(rel)) {
-    G.ctl[kCtlStatus] = NW_NAN_DETECTED;
-    G.ctl[kCtlBasis] = j + 1;
-    G.ctl[kCtlDone] = 1;
-  } else if (rel <= c.tol || hn == 0.0) {
-    G.ctl[kCtlBasis] = j + 1;
-    G.ctl[kCtlDone] = 1;
-  }
-}
-
 // v = w / nrm[0] and, when rd is given, z = rd * v (the Jacobi application
-// of the next Arnoldi step) in the same pass. GIVENS: block 0 instead applies
-// the Givens rotations to the new Hessenberg column, beside the scaling.
+// of the next Arnoldi step) in the same pass. GIVENS: block 0 instead forms
+// the new column's Givens rotation, beside the scaling.
 template <typename T, bool GIVENS>
 __global__ void __launch_bounds__(kBlock)
     scale_jacobi_k(int64_t n, const T* __restrict__ w, T* __restrict__ v, const double* __restrict__ nrm,
                    const T* __restrict__ rd, T* __restrict__ z, GivensCol gc) {
   if (GIVENS && blockIdx.x == 0) {
-    if (threadIdx.x < 32) givens_step(gc);
+    if (threadIdx.x == 0) givens_finish(gc);
     return;
   }
   __shared__ T inv;
@@ -1419,17 +1427,23 @@ void KrylovSolver::mdot64(int nv, const double* V, int64_t ld, const double* w, 
   }
 }
 
-// w -= sum_k h[k] V[k]; with nrm also nrm[0] = ||w||
+// w -= sum_k h[k] V[k]; with nrm also nrm[0] = ||w||; with gc the earlier
+// rotations of that column
 void KrylovSolver::maxpy64(int nv, const double* V, int64_t ld, const double* h, double* w, double* nrm,
-                           cudaStream_t s) {
+                           cudaStream_t s, const GivensCol* gc) {
   const int64_t n = A_.n;
-  const unsigned g = grid1(n);
+  const unsigned g = grid1(n), rot = gc ? 1 : 0;
+  const GivensDev G = gc ? gc->G : GivensDev{};
+  auto launch = [&](auto kernel, unsigned ept) {
+    kernel<<<(g + ept - 1) / ept + rot, kBlock, 0, s>>>(n, nv, V, ld, h, w, partial_.p, nrm, ticket_.p, G,
+                                                        gc ? gc->j : 0, gc ? gc->hs : nullptr);
+  };
   if (g >= unsigned(8 * 3 * sms_))
-    maxpy64_k<8><<<(g + 7) / 8, kBlock, 0, s>>>(n, nv, V, ld, h, w, partial_.p, nrm, ticket_.p);
+    launch(maxpy64_k<8>, 8);
   else if (g >= unsigned(4 * sms_))
-    maxpy64_k<4><<<(g + 3) / 4, kBlock, 0, s>>>(n, nv, V, ld, h, w, partial_.p, nrm, ticket_.p);
+    launch(maxpy64_k<4>, 4);
   else
-    maxpy64_k<1><<<g, kBlock, 0, s>>>(n, nv, V, ld, h, w, partial_.p, nrm, ticket_.p);
+    launch(maxpy64_k<1>, 1);
 }
 
 double KrylovSolver::dot(const double* a, const double* b, cudaStream_t s) {
@@ -1936,7 +1950,7 @@ SolveResult KrylovSolver::gmres(const nw_solver_cfg& cfg, double tol,
       mdot64(j + 1, V, n, w_.p, hs, nullptr, s);
       maxpy64(j + 1, V, n, hs, w_.p, nullptr, s);
       mdot64(j + 1, V, n, w_.p, h2 + 1, hs, s);
-      maxpy64(j + 1, V, n, h2 + 1, w_.p, h2, s);
+      maxpy64(j + 1, V, n, h2 + 1, w_.p, h2, s, &gc);
       double* znext = (j + 1 < m) ? (flexible ? Z_.p + size_t(j + 1) * n : z_.p) : nullptr;
       scale_jacobi_k<double, true><<<grid1(n) + 1, kBlock, 0, s>>>(
           n, w_.p, V + size_t(j + 1) * n, h2, (fuse_jacobi && znext) ? rdiag_.p : nullptr, znext, gc);
@@ -2491,7 +2505,7 @@ SolveResult KrylovSolver::mixed(const nw_solver_cfg& cfg, double tol,
       // second pass of the FP64 method is not needed here (same iteration
       // counts on the Poisson systems measured)
       mdot4_k<<<dim3(mdot4_blocks_, j / kTile + 1), kBlock, 0, s>>>(n, j + 1, V, ld, w32_.p, partial_.p, hs, ticket_.p);
-      maxpy4_k<<<g4, kBlock, 0, s>>>(n, j + 1, V, ld, hs, w32_.p, partial_.p, h2, ticket_.p);
+      maxpy4_k<<<g4 + 1, kBlock, 0, s>>>(n, j + 1, V, ld, hs, w32_.p, partial_.p, h2, ticket_.p, gc.G, j);
       scale_jacobi_k<float, true><<<grid1(n) + 1, kBlock, 0, s>>>(n, w32_.p, V + size_t(j + 1) * ld, h2,
                                                                   fuse_jacobi ? rdiag32_.p : nullptr, z32_.p, gc);
     };

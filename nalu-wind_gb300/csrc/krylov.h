@@ -52,6 +52,27 @@ struct SolveResult {
   std::vector<double> history;
 };
 
+// GMRES least squares on the device (krylov.cu): the rotated Hessenberg
+// columns, the rotations, the rotated rhs, the residual estimates and the
+// control words.
+struct GivensDev {
+  double *H, *cs, *sn, *g, *hist;
+  int* ctl;
+  int m;
+};
+enum { kCtlDone = 0, kCtlIts = 1, kCtlStatus = 2, kCtlBasis = 3 };  // kCtlIts: of the cycle
+
+// Column j: h = hs[0..j], hn = ||w||. rel = |g[j+1]| / div; the history
+// entry is rel * hist_mul / hist_div; the cycle stops when rel <= tol or
+// hn == 0 (basis j + 1), on a non-finite estimate (basis j + 1) or when the
+// rotation breaks down (basis j).
+struct GivensCol {
+  GivensDev G;
+  int j;
+  const double *hs, *hn;
+  double tol, div, hist_mul, hist_div;
+};
+
 class KrylovSolver {
  public:
   KrylovSolver() = default;
@@ -207,7 +228,8 @@ class KrylovSolver {
   int64_t ld32_ = 0;  // leading dimension of the FP32 basis (n rounded up to 32)
   bool f32_valid_ = false;
   void mdot64(int nv, const double* V, int64_t ld, const double* w, double* out, double* acc, cudaStream_t s);
-  void maxpy64(int nv, const double* V, int64_t ld, const double* h, double* w, double* nrm, cudaStream_t s);
+  void maxpy64(int nv, const double* V, int64_t ld, const double* h, double* w, double* nrm, cudaStream_t s,
+               const GivensCol* gc = nullptr);
   DeviceArray<int> ticket_;   // finished blocks per tile of a reduction (zero between launches)
   int sms_ = 1;
   int red_blocks_ = 0;
