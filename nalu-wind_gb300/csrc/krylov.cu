@@ -1110,7 +1110,10 @@ __global__ void __launch_bounds__(kBlock)
     scale_jacobi_k(int64_t n, const T* __restrict__ w, T* __restrict__ v, const double* __restrict__ nrm,
                    const T* __restrict__ rd, T* __restrict__ z, GivensCol gc) {
   if (GIVENS && blockIdx.x == 0) {
-    if (threadIdx.x == 0) givens_finish(gc);
+    if (threadIdx.x == 0) {
+      givens_finish(gc);
+      if (gc.poll) *reinterpret_cast<int4*>(gc.poll) = *reinterpret_cast<const int4*>(gc.G.ctl);
+    }
     return;
   }
   __shared__ T inv;
@@ -1156,8 +1159,8 @@ template <typename StepFn>
 KrylovSolver::Cycle KrylovSolver::run_cycle(int m, int max_steps, double g0, double tol, double div,
                                             double hist_mul, double hist_div, StepFn arnoldi,
                                             const double* hs, const double* hn, cudaStream_t s,
-                                            bool graph) {
-  constexpr int kChunk = 2;  // iterations per poll; the host waits one chunk behind
+                                            bool graph, bool set_up) {
+  constexpr int kChunk = 2;  // iterations per poll and per graph; the host waits one chunk behind
   GivensDev G{gst_.p,
               gst_.p + size_t(m_ + 1) * m_,
               gst_.p + size_t(m_ + 1) * m_ + m_,
@@ -1167,19 +1170,27 @@ KrylovSolver::Cycle KrylovSolver::run_cycle(int m, int max_steps, double g0, dou
   givens_init_k<<<1, 32, 0, s>>>(G, g0);
   int launched = 0, pending = -1, slot = 0;
   bool stop = false;
-  auto step = [&](int j) { arnoldi(j, GivensCol{G, j, hs, hn, tol, div, hist_mul, hist_div}); };
-  for (int j = 0; j < m && launched < max_steps && !stop; ++j) {
-    // the first step of a cycle runs as plain launches: any one-time set-up
-    // (buffer growth) happens there, outside a capture. A stream that cannot
-    // be captured (the legacy default stream) keeps plain launches.
-    if (graph && j > 0 && cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
+  for (int j = 0; j < m && launched < max_steps && !stop;) {
+    const int cnt = std::min({kChunk, m - j, max_steps - launched});
+    const bool full = cnt == kChunk;
+    auto chunk = [&] {
+      for (int k = 0; k < cnt; ++k)
+        arnoldi(j + k, GivensCol{G, j + k, hs, hn, tol, div, hist_mul, hist_div,
+                                 full && k == cnt - 1 ? ctl_pinned_ + 4 * slot : nullptr});
+    };
+    // A solve's first chunk runs as plain launches: any one-time set-up
+    // (buffer growth) happens there, outside a capture. So does a shorter
+    // last chunk, which would not fit the graph, and every chunk on a stream
+    // that cannot be captured (the legacy default stream).
+    bool captured = graph && full && (set_up || j > 0);
+    if (captured && cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
       cudaGetLastError();
-      graph = false;
+      graph = captured = false;
     }
-    if (graph && j > 0) {
+    if (captured) {
       cudaGraph_t g = nullptr;
       try {
-        step(j);
+        chunk();
       } catch (...) {
         cudaStreamEndCapture(s, &g);
         if (g) cudaGraphDestroy(g);
@@ -1205,11 +1216,11 @@ KrylovSolver::Cycle KrylovSolver::run_cycle(int m, int max_steps, double g0, dou
       cudaGraphDestroy(g);
       NW_CUDA(cudaGraphLaunch(iter_exec_, s));
     } else {
-      step(j);
+      chunk();
     }
-    ++launched;
-    if (launched % kChunk == 0) {
-      NW_CUDA(cudaMemcpyAsync(ctl_pinned_ + 4 * slot, gctl_.p, 4 * sizeof(int), cudaMemcpyDeviceToHost, s));
+    j += cnt;
+    launched += cnt;
+    if (full) {
       NW_CUDA(cudaEventRecord(chunk_ev_[slot], s));
       if (pending >= 0) {
         NW_CUDA(cudaEventSynchronize(chunk_ev_[pending]));
@@ -1955,7 +1966,8 @@ SolveResult KrylovSolver::gmres(const nw_solver_cfg& cfg, double tol,
       scale_jacobi_k<double, true><<<grid1(n) + 1, kBlock, 0, s>>>(
           n, w_.p, V + size_t(j + 1) * n, h2, (fuse_jacobi && znext) ? rdiag_.p : nullptr, znext, gc);
     };
-    const Cycle c = run_cycle(m, cfg.max_iterations - its, beta, tol, bnorm, 1.0, 1.0, arnoldi, hs, h2, s);
+    const Cycle c = run_cycle(m, cfg.max_iterations - its, beta, tol, bnorm, 1.0, 1.0, arnoldi, hs, h2, s,
+                              !pc.apply_fn, its > 0);
     its += c.iterations;
     res.history.insert(res.history.end(), c.hist.begin(), c.hist.end());
     if (!c.hist.empty()) rel = c.hist.back();
@@ -2510,7 +2522,7 @@ SolveResult KrylovSolver::mixed(const nw_solver_cfg& cfg, double tol,
                                                                   fuse_jacobi ? rdiag32_.p : nullptr, z32_.p, gc);
     };
     const Cycle c = run_cycle(m, cfg.max_iterations - its, 1.0, itol, 1.0, rnorm, bnorm, arnoldi, hs, h2, s,
-                              true);
+                              true, its > 0);
     its += c.iterations;
     res.history.insert(res.history.end(), c.hist.begin(), c.hist.end());
     if (c.status != NW_OK) res.status = c.status;

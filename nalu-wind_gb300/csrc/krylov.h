@@ -71,6 +71,7 @@ struct GivensCol {
   int j;
   const double *hs, *hn;
   double tol, div, hist_mul, hist_div;
+  int* poll;  // pinned host copy of the control words, or null
 };
 
 class KrylovSolver {
@@ -151,7 +152,7 @@ class KrylovSolver {
   // control words done, iterations of the cycle, status, basis size.
   DeviceArray<double> gst_;
   DeviceArray<int> gctl_;
-  int* ctl_pinned_ = nullptr;   // host mirrors of gctl_ (3 slots)
+  int* ctl_pinned_ = nullptr;   // copies of gctl_: two the device writes, one copied
   cudaEvent_t chunk_ev_[2] = {nullptr, nullptr};
   struct Cycle {
     int iterations = 0;  // rotations applied (iterations counted)
@@ -164,13 +165,13 @@ class KrylovSolver {
   // j's kernels: the new column in hs[0..j], its norm at hn[0], then the
   // column's Givens update beside the scaling of the new vector), with the
   // host one chunk behind.
-  // With `graph`, the steps after the first of the cycle are captured from
-  // the same launches into a CUDA graph each, which updates iter_exec_ in
-  // place and is launched as one unit (the kernels then follow each other
-  // without the per-launch gaps of a stream).
+  // With `graph`, chunks after the solve's first (set_up: an earlier cycle has
+  // run) are captured from the same launches into a CUDA graph each, which
+  // updates iter_exec_ in place and is launched as one unit (the kernels then
+  // follow each other without the per-launch gaps of a stream).
   template <typename StepFn>
   Cycle run_cycle(int m, int max_steps, double g0, double tol, double div, double hist_mul, double hist_div,
-                  StepFn arnoldi, const double* hs, const double* hn, cudaStream_t s, bool graph = false);
+                  StepFn arnoldi, const double* hs, const double* hn, cudaStream_t s, bool graph, bool set_up);
   cudaGraphExec_t iter_exec_ = nullptr;
   // Sliced ELLPACK copy (slices of 32 rows, column-major within a slice)
   // used by the solver's SpMV: coalesced value/column loads for short rows.
