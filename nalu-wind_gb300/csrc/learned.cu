@@ -22,6 +22,7 @@
 #include <fstream>
 #include <numeric>
 
+#include "last_block.h"
 #include "learned.h"
 
 namespace nw {
@@ -220,9 +221,15 @@ __global__ void colsum_k(int nblocks, int ncols, const float* __restrict__ parti
   dst[j] = accumulate ? dst[j] + s : s;
 }
 
+constexpr int kAggBatch = 32;  // gathers in flight
+
 // ---------------------------------------------------------------------------
 // Aggregation over the coarse graph (diagonal slot skipped):
 // out[I][64 + c] = sum_J w_IJ in[J][c], in/out BF16 with row stride 128.
+// Bound by the latency of the gathered rows: the lanes load a row's columns
+// and weights together and up to 32 gathers are in flight, then the
+// multiply-adds in column order: 1,216 rows take 3.8 us, 5.0 with one load,
+// gather and multiply-add after the other.
 __global__ void __launch_bounds__(kB)
     agg_fwd_k(int64_t nc, const int64_t* __restrict__ cptr,
               const int32_t* __restrict__ ccol, const int32_t* __restrict__ cdiag,
@@ -231,13 +238,29 @@ __global__ void __launch_bounds__(kB)
   const int lane = threadIdx.x & 31;
   if (I >= nc) return;
   float a0 = 0.f, a1 = 0.f;
-  const int64_t dpos = cdiag[I];
-  for (int64_t q = cptr[I]; q < cptr[I + 1]; ++q) {
-    if (q == dpos) continue;
-    const float w = wgt[q];
-    const uint32_t v = *reinterpret_cast<const uint32_t*>(xc + int64_t(ccol[q]) * 128 + 2 * lane);
-    a0 = fmaf(w, bf2f(uint16_t(v & 0xffffu)), a0);
-    a1 = fmaf(w, bf2f(uint16_t(v >> 16)), a1);
+  const int64_t dpos = cdiag[I], q1 = cptr[I + 1];
+  for (int64_t q = cptr[I]; q < q1; q += 32) {
+    const bool on = q + lane < q1 && q + lane != dpos;
+    const int32_t c = on ? ccol[q + lane] : -1;
+    const float w = on ? wgt[q + lane] : 0.f;
+    const int cnt = int(min(int64_t(32), q1 - q));
+    for (int j = 0; j < cnt; j += kAggBatch) {
+      uint32_t v[kAggBatch];
+      int32_t cj[kAggBatch];
+#pragma unroll
+      for (int k = 0; k < kAggBatch; ++k) {
+        cj[k] = __shfl_sync(0xffffffffu, c, j + k);
+        v[k] = cj[k] >= 0 ? *reinterpret_cast<const uint32_t*>(xc + int64_t(cj[k]) * 128 + 2 * lane) : 0u;
+      }
+#pragma unroll
+      for (int k = 0; k < kAggBatch; ++k) {
+        const float wk = __shfl_sync(0xffffffffu, w, j + k);
+        if (cj[k] >= 0) {
+          a0 = fmaf(wk, bf2f(uint16_t(v[k] & 0xffffu)), a0);
+          a1 = fmaf(wk, bf2f(uint16_t(v[k] >> 16)), a1);
+        }
+      }
+    }
   }
   *reinterpret_cast<uint32_t*>(xc + I * 128 + 64 + 2 * lane) = pack2(f2bf(a0), f2bf(a1));
 }
@@ -276,10 +299,43 @@ __global__ void mask_k(int64_t nc, const float* __restrict__ dh,
   dz[q] = f2bf(bf2f(h[I * ldh + c]) > 0.f ? dh[q] : 0.f);
 }
 
-// u = rc * dinv; partial sums of u^2
-__global__ void input_k(int64_t nc, const float* __restrict__ rc,
-                        const float* __restrict__ dinv, float* __restrict__ u,
-                        float* __restrict__ partial) {
+// Fixed-order sums of part(b, w), b < nblocks, for w < W, by one block of kB
+// threads: strided per-thread sums, then a tree over the threads; results
+// in thread 0. Threads without a partial hold an exact zero, so the levels that
+// would only add those are left out, and the last ones run in the first warp's
+// registers.
+template <int W, typename F>
+__device__ __forceinline__ void block_sum(int nblocks, double (&v)[W], F part) {
+  __shared__ double red[W][kB];
+  const int t = threadIdx.x;
+#pragma unroll
+  for (int w = 0; w < W; ++w) v[w] = 0.0;
+  for (int b = t; b < nblocks; b += kB)
+#pragma unroll
+    for (int w = 0; w < W; ++w) v[w] += part(b, w);
+  int h = kB / 2;
+  while (h >= nblocks && h > 1) h >>= 1;
+  if (h >= 32) {
+#pragma unroll
+    for (int w = 0; w < W; ++w) red[w][t] = v[w];
+    __syncthreads();
+    for (; h >= 32; h >>= 1) {
+      if (t < h)
+#pragma unroll
+        for (int w = 0; w < W; ++w) red[w][t] = v[w] = v[w] + red[w][t + h];
+      __syncthreads();
+    }
+  }
+  for (; h > 0; h >>= 1)
+#pragma unroll
+    for (int w = 0; w < W; ++w) v[w] += __shfl_down_sync(0xffffffffu, v[w], h);
+}
+
+// u = rc * dinv and its scale: scal[0] = s = sqrt(sum u^2 / nc), scal[1] = 1/s
+// (0 when s == 0) from the per-block sums, by the last block
+__global__ void __launch_bounds__(kB)
+    input_k(int64_t nc, const float* __restrict__ rc, const float* __restrict__ dinv, float* __restrict__ u,
+            float* partial, float* __restrict__ scal, int* __restrict__ ticket) {
   __shared__ float red[kB / 32];
   const int64_t I = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   float v = 0.f;
@@ -296,32 +352,11 @@ __global__ void input_k(int64_t nc, const float* __restrict__ rc,
     for (int q = 0; q < kB / 32; ++q) t += red[q];
     partial[blockIdx.x] = t;
   }
-}
-
-// Fixed-order sum of partial[b * stride + which], b < nblocks, by one block
-// of kB threads (strided per-thread sums, then a tree).
-__device__ double block_sum(int nblocks, const float* __restrict__ partial, int stride, int which,
-                            double* red) {
-  double t = 0.0;
-  for (int b = threadIdx.x; b < nblocks; b += kB) t += partial[int64_t(b) * stride + which];
-  red[threadIdx.x] = t;
-  __syncthreads();
-  for (int h = kB / 2; h > 0; h >>= 1) {
-    if (threadIdx.x < h) red[threadIdx.x] += red[threadIdx.x + h];
-    __syncthreads();
-  }
-  const double v = red[0];
-  __syncthreads();
-  return v;
-}
-
-// scal[0] = s = sqrt(sum u^2 / nc), scal[1] = 1 / s (0 when s == 0)
-__global__ void __launch_bounds__(kB)
-    rms_k(int nblocks, const float* __restrict__ partial, int64_t nc, float* __restrict__ scal) {
-  __shared__ double red[kB];
-  const double t = block_sum(nblocks, partial, 1, 0, red);
+  if (!last_block(ticket, gridDim.x)) return;
+  double t[1];
+  block_sum<1>(gridDim.x, t, [&](int b, int) { return __ldcg(partial + b); });
   if (threadIdx.x == 0) {
-    const double s = std::sqrt(t / double(nc > 0 ? nc : 1));
+    const double s = std::sqrt(t[0] / double(nc > 0 ? nc : 1));
     scal[0] = float(s);
     scal[1] = s > 0 ? float(1.0 / s) : 0.f;
   }
@@ -371,9 +406,6 @@ __global__ void __launch_bounds__(kB)
   }
 }
 
-// Coarse operator applied to the network output, thread per coarse row:
-//   (Ac ec)_I = (ec_I - sum_J w_IJ ec_J) / dinv_I     (Ac = D (I - W))
-// with per-block partial sums of ec' rc and ec' Ac ec (two per block).
 // Jacobi step on the coarse operator, written with w_IJ = -Ac_IJ / Ac_II
 // and dinv = 1 / Ac_II: e_out = dinv r + sum_J w_IJ e_in,J (e_in == nullptr:
 // e_out = dinv r, the step from zero).
@@ -393,56 +425,94 @@ __global__ void coarse_jacobi_k(int64_t nc, const int64_t* __restrict__ cptr,
   eout[I] = v;
 }
 
-__global__ void coarse_apply_k(int64_t nc, const int64_t* __restrict__ cptr,
-                               const int32_t* __restrict__ ccol,
-                               const int32_t* __restrict__ cdiag,
-                               const float* __restrict__ wgt, const float* __restrict__ dinv,
-                               const float* __restrict__ ec, const float* __restrict__ rc,
-                               float* __restrict__ aec, float* __restrict__ partial) {
-  __shared__ float red[2][kB / 32];
-  const int64_t I = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  float num = 0.f, den = 0.f;
-  if (I < nc) {
-    const float e = ec[I];
-    float a = e;
-    const int64_t dpos = cdiag[I];
-    for (int64_t q = cptr[I]; q < cptr[I + 1]; ++q)
-      if (q != dpos) a = fmaf(-wgt[q], ec[ccol[q]], a);
-    const float d = dinv[I];
-    const float v = d != 0.f ? a / d : 0.f;
-    aec[I] = v;
-    num = e * rc[I];
-    den = e * v;
-  }
-  for (int off = 16; off > 0; off >>= 1) {
-    num += __shfl_down_sync(0xffffffffu, num, off);
-    den += __shfl_down_sync(0xffffffffu, den, off);
-  }
-  if ((threadIdx.x & 31) == 0) {
-    red[0][threadIdx.x >> 5] = num;
-    red[1][threadIdx.x >> 5] = den;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float a = 0.f, b = 0.f;
-    for (int q = 0; q < kB / 32; ++q) {
-      a += red[0][q];
-      b += red[1][q];
-    }
-    partial[2 * blockIdx.x] = a;
-    partial[2 * blockIdx.x + 1] = b;
-  }
-}
-
-// Energy-optimal scaling of the coarse correction, fixed-order sums:
+// Coarse operator applied to the network output:
+//   (Ac ec)_I = (ec_I - sum_J w_IJ ec_J) / dinv_I     (Ac = D (I - W))
+// with partial sums of ec' rc and ec' Ac ec (two per 32 rows), and in the last
+// block the energy-optimal scaling of the coarse correction from their
+// fixed-order sums (per 256 rows, then those):
 //   scal[2] = alpha = ec' rc / ec' Ac ec   (0 unless the denominator is > 0)
 //   scal[3] = (ec' rc)^2 / ec' Ac ec       (A-norm error energy removed)
-__global__ void __launch_bounds__(kB)
-    alpha_k(int nblocks, const float* __restrict__ partial, float* __restrict__ scal) {
-  __shared__ double red[kB];
-  const double num = block_sum(nblocks, partial, 2, 0, red);
-  const double den = block_sum(nblocks, partial, 2, 1, red);
+//
+// Bound by latency: some thousand coarse rows of about 27 entries. kRowLanes
+// lanes share a row, so that its columns, weights and gathered values are
+// loaded side by side; the multiply-adds follow in column order on every lane.
+// With the scaling's launch of its own, 1,216 rows took 8.9 us with a thread a
+// row, 5.7 now.
+constexpr int kRowLanes = 8, kRowBlock = 32;
+__global__ void __launch_bounds__(kRowLanes * kRowBlock)
+    coarse_apply_k(int64_t nc, const int64_t* __restrict__ cptr,
+                   const int32_t* __restrict__ ccol,
+                   const int32_t* __restrict__ cdiag,
+                   const float* __restrict__ wgt, const float* __restrict__ dinv,
+                   const float* __restrict__ ec, const float* __restrict__ rc,
+                   float* __restrict__ aec, float* partial, float* __restrict__ scal,
+                   int* __restrict__ ticket) {
+  __shared__ float red[2][kRowBlock];
+  const int row = threadIdx.x / kRowLanes, sub = threadIdx.x % kRowLanes;
+  const int64_t I = int64_t(blockIdx.x) * kRowBlock + row;
+  const unsigned lanes = ((1u << kRowLanes) - 1) << (threadIdx.x % 32 - sub);
+  float num = 0.f, den = 0.f;
+  if (I < nc) {
+    constexpr int B = 4;
+    const float e = ec[I], r = rc[I], d = dinv[I];
+    float a = e;
+    const int64_t dpos = cdiag[I], q1 = cptr[I + 1];
+    for (int64_t q = cptr[I]; q < q1; q += B * kRowLanes) {
+      int32_t c[B];
+      float w[B], ej[B];
+#pragma unroll
+      for (int j = 0; j < B; ++j) {
+        const int64_t p = q + j * kRowLanes + sub;
+        const bool on = p < q1 && p != dpos;
+        c[j] = on ? ccol[p] : -1;
+        w[j] = on ? wgt[p] : 0.f;
+      }
+#pragma unroll
+      for (int j = 0; j < B; ++j) ej[j] = c[j] >= 0 ? ec[c[j]] : 0.f;
+#pragma unroll
+      for (int j = 0; j < B; ++j)
+#pragma unroll
+        for (int k = 0; k < kRowLanes; ++k) {
+          const float wk = __shfl_sync(lanes, w[j], k, kRowLanes), ek = __shfl_sync(lanes, ej[j], k, kRowLanes);
+          if (__shfl_sync(lanes, c[j], k, kRowLanes) >= 0) a = fmaf(-wk, ek, a);
+        }
+    }
+    const float v = d != 0.f ? a / d : 0.f;
+    if (sub == 0) aec[I] = v;
+    num = e * r;
+    den = e * v;
+  }
+  if (sub == 0) {
+    red[0][row] = num;
+    red[1][row] = den;
+  }
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    num = red[0][threadIdx.x];
+    den = red[1][threadIdx.x];
+    for (int off = 16; off > 0; off >>= 1) {
+      num += __shfl_down_sync(0xffffffffu, num, off);
+      den += __shfl_down_sync(0xffffffffu, den, off);
+    }
+    if (threadIdx.x == 0) {
+      partial[2 * blockIdx.x] = num;
+      partial[2 * blockIdx.x + 1] = den;
+    }
+  }
+  if (!last_block(ticket, gridDim.x)) return;
+  // per 256 rows: their eight sums in order, in single precision
+  const int nb32 = int(gridDim.x), nb = (nb32 + 7) / 8;
+  double t[2];
+  block_sum<2>(nb, t, [&](int b, int w) {
+    float x[8], v = 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) x[k] = 8 * b + k < nb32 ? __ldcg(partial + 2 * (8 * b + k) + w) : 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v += x[k];
+    return v;
+  });
   if (threadIdx.x == 0) {
+    const double num = t[0], den = t[1];
     const bool ok = den > 0.0 && isfinite(num) && isfinite(den);
     scal[2] = ok ? float(num / den) : 0.f;
     scal[3] = ok ? float(num * num / den) : 0.f;
@@ -871,8 +941,13 @@ void CoarseLevel::refresh(const double* fine_values, cudaStream_t s) {
   NW_CUDA(cudaGetLastError());
 }
 
-void NetWork::resize(int64_t n) {
+void NetWork::resize(int64_t n, cudaStream_t s) {
   if (n == nc && u.p) return;
+  if (!ticket.p) {
+    ticket.resize(1);
+    NW_CUDA(cudaMemsetAsync(ticket.p, 0, sizeof(int), s));
+    NW_CUDA(cudaStreamSynchronize(s));
+  }
   nc = n;
   u.resize(n);
   x.resize(n);
@@ -880,7 +955,7 @@ void NetWork::resize(int64_t n) {
   y.resize(n);
   dy.resize(n);
   scal.resize(4);
-  partial.resize(2 * gridn(n) + 2);
+  partial.resize(2 * gridn(n, 32) + 2);
   aec.resize(n);
   ec.resize(n);
   part2.resize(size_t(gridn(n * 64)) * 128);
@@ -954,10 +1029,9 @@ void LearnedNet::clear_data() {
 void LearnedNet::forward(const CoarseLevel& cl, const float* wgt, const float* dinv,
                          const float* rc, float* ec, cudaStream_t s) {
   const int64_t nc = cl.nc;
-  work.resize(nc);
+  work.resize(nc, s);
   const unsigned gw = gridn(nc * 32);  // warp per row
-  input_k<<<gridn(nc), kB, 0, s>>>(nc, rc, dinv, work.u.p, work.partial.p);
-  rms_k<<<1, kB, 0, s>>>(int(gridn(nc)), work.partial.p, nc, work.scal.p);
+  input_k<<<gridn(nc), kB, 0, s>>>(nc, rc, dinv, work.u.p, work.partial.p, work.scal.p, work.ticket.p);
   layer0_k<<<gw, kB, 0, s>>>(nc, cl.cptr.p, cl.ccol.p, cl.cdiag.p, wgt, work.u.p, work.scal.p,
                              params.p + kOffW0, work.x.p, work.ax.p, work.xc1.p);
   uint16_t* xcs[4] = {work.xc1.p, work.xc2.p, work.xc3.p, nullptr};
@@ -976,16 +1050,15 @@ void LearnedNet::coarse_correction(const CoarseLevel& cl, const float* rc, float
   if (coarse_mode == 0) {
     forward(cl, cl.wgt.p, cl.dinv.p, rc, ec, s);
   } else {
-    work.resize(cl.nc);
+    work.resize(cl.nc, s);
     coarse_jacobi_k<<<nb, kB, 0, s>>>(cl.nc, cl.cptr.p, cl.ccol.p, cl.cdiag.p, cl.wgt.p, cl.dinv.p, rc,
                                       nullptr, coarse_mode == 1 ? ec : work.u.p);
     if (coarse_mode == 2)
       coarse_jacobi_k<<<nb, kB, 0, s>>>(cl.nc, cl.cptr.p, cl.ccol.p, cl.cdiag.p, cl.wgt.p, cl.dinv.p, rc,
                                         work.u.p, ec);
   }
-  coarse_apply_k<<<nb, kB, 0, s>>>(cl.nc, cl.cptr.p, cl.ccol.p, cl.cdiag.p, cl.wgt.p, cl.dinv.p,
-                                   ec, rc, work.aec.p, work.partial.p);
-  alpha_k<<<1, kB, 0, s>>>(nb, work.partial.p, work.scal.p);
+  coarse_apply_k<<<gridn(cl.nc, kRowBlock), kB, 0, s>>>(cl.nc, cl.cptr.p, cl.ccol.p, cl.cdiag.p, cl.wgt.p, cl.dinv.p,
+                                   ec, rc, work.aec.p, work.partial.p, work.scal.p, work.ticket.p);
   NW_CUDA(cudaGetLastError());
 }
 
@@ -993,14 +1066,13 @@ double LearnedNet::forward_backward(const CoarseLevel& cl, const float* wgt,
                                     const float* dinv, const float* rc, double ea,
                                     double ca, cudaStream_t s, bool with_grad) {
   const int64_t nc = cl.nc;
-  work.resize(nc);
+  work.resize(nc, s);
   float* ec = work.ec.p;
   forward(cl, wgt, dinv, rc, ec, s);
   const unsigned gw = gridn(nc * 32);
   const int nb = int(gridn(nc));
-  coarse_apply_k<<<nb, kB, 0, s>>>(nc, cl.cptr.p, cl.ccol.p, cl.cdiag.p, wgt, dinv, ec, rc,
-                                   work.aec.p, work.partial.p);
-  alpha_k<<<1, kB, 0, s>>>(nb, work.partial.p, work.scal.p);
+  coarse_apply_k<<<gridn(nc, kRowBlock), kB, 0, s>>>(nc, cl.cptr.p, cl.ccol.p, cl.cdiag.p, wgt, dinv, ec, rc,
+                                   work.aec.p, work.partial.p, work.scal.p, work.ticket.p);
   float sc[4];
   NW_CUDA(cudaMemcpyAsync(sc, work.scal.p, sizeof(sc), cudaMemcpyDeviceToHost, s));
   NW_CUDA(cudaStreamSynchronize(s));

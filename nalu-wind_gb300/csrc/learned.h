@@ -77,7 +77,8 @@ struct NetWork {
   DeviceArray<float> u, x, ax, y, dy, ec, aec, scal, partial, part2;
   DeviceArray<uint16_t> xc1, xc2, xc3, h3, dz;  // BF16
   DeviceArray<float> dxc, dh;
-  void resize(int64_t n);
+  DeviceArray<int> ticket;  // finished blocks of a reduction (zero between launches)
+  void resize(int64_t n, cudaStream_t s);
 };
 
 struct LearnedNet {
