@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(kBlock)
   if (row < n) y[row] = b ? XT(ACC(b[row]) - acc) : XT(acc);
 }
 
-// values in SELL order (FP64 and optionally FP32) from the CSR values
+// values in SELL order (FP64 and / or FP32) from the CSR values
 __global__ void sell_gather_k(int64_t slots, const int32_t* __restrict__ map,
                               const double* __restrict__ csr,
                               double* __restrict__ out64, float* __restrict__ out32) {
@@ -161,7 +161,7 @@ __global__ void sell_gather_k(int64_t slots, const int32_t* __restrict__ map,
   if (q >= slots) return;
   const int32_t p = map[q];
   const double v = p >= 0 ? csr[p] : 0.0;
-  out64[q] = v;
+  if (out64) out64[q] = v;
   if (out32) out32[q] = float(v);
 }
 
@@ -916,7 +916,7 @@ __global__ void rdiag_k(int64_t n, const int64_t* __restrict__ rp,
   double d = 0.0;
   for (int64_t p = rp[i]; p < rp[i + 1]; ++p)
     if (ci[p] == i) d = v[p];
-  rd[i] = 1.0 / d;
+  if (rd) rd[i] = 1.0 / d;
   if (d32) d32[i] = float(d);
 }
 
@@ -1333,7 +1333,7 @@ void KrylovSolver::refresh(cudaStream_t s) {
   NW_CUDA(cudaGetLastError());
   f32_valid_ = false;
   ilu_valid_ = false;
-  gs_vals16_.release();
+  bf16_valid_ = false;
 }
 
 void KrylovSolver::ensure_f32(cudaStream_t s) {
@@ -1351,7 +1351,7 @@ void KrylovSolver::ensure_f32(cudaStream_t s) {
   if (sell_slices_) {
     sell_vals32_.resize(sell_vals_.n);
     sell_gather_k<<<grid1(int64_t(sell_vals_.n)), kBlock, 0, s>>>(
-        int64_t(sell_vals_.n), sell_map_.p, A_.values, sell_vals_.p, sell_vals32_.p);
+        int64_t(sell_vals_.n), sell_map_.p, A_.values, nullptr, sell_vals32_.p);
   }
   if (gs_map_.n) {
     gs_vals32_.resize(gs_map_.n);
@@ -1360,14 +1360,21 @@ void KrylovSolver::ensure_f32(cudaStream_t s) {
   }
   convert_k<double, float><<<grid1(n), kBlock, 0, s>>>(n, rdiag_.p, rdiag32_.p);
   diag32_.resize(n);
-  {
-    DeviceArray<double> tmp;
-    tmp.resize(n);
-    rdiag_k<<<grid1(n), kBlock, 0, s>>>(n, A_.row_ptr, A_.col_idx, A_.values, tmp.p, diag32_.p);
-    NW_CUDA(cudaStreamSynchronize(s));
-  }
+  rdiag_k<<<grid1(n), kBlock, 0, s>>>(n, A_.row_ptr, A_.col_idx, A_.values, nullptr, diag32_.p);
   NW_CUDA(cudaGetLastError());
   f32_valid_ = true;
+}
+
+// BF16 copy of the Gauss-Seidel values, kept between solves like the FP32 ones
+// (freed and allocated for each it held the stream up for 0.13 ms a solve)
+void KrylovSolver::ensure_bf16(cudaStream_t s) {
+  if (bf16_valid_) return;
+  gs_vals16_.resize(gs_vals32_.n);
+  if (gs_vals32_.n)
+    to_bf16_vals_k<<<grid1(int64_t(gs_vals32_.n)), kBlock, 0, s>>>(int64_t(gs_vals32_.n), gs_vals32_.p,
+                                                                  gs_vals16_.p);
+  NW_CUDA(cudaGetLastError());
+  bf16_valid_ = true;
 }
 
 void KrylovSolver::spmv(const double* x, double* y, cudaStream_t s) const {
@@ -1629,6 +1636,7 @@ void KrylovSolver::setup_colors(const std::vector<int32_t>& rows,
   gs_vals_.resize(std::max<int64_t>(off[ns], 1));
   gs_vals32_.release();
   f32_valid_ = false;
+  bf16_valid_ = false;
 }
 
 // Pre-smoothing of the learned cycle (also used when harvesting pairs):
@@ -1636,6 +1644,7 @@ void KrylovSolver::setup_colors(const std::vector<int32_t>& rows,
 void KrylovSolver::learned_presmooth32(const float* x, float* y, cudaStream_t s) {
   if (!has_learned()) fail(NW_INVALID_ARG, "no learned preconditioner attached");
   ensure_f32(s);
+  if (gs_bf16_) ensure_bf16(s);
   const int sweep = net_->smoother == 1 ? 1 : 0;
   if (gs_bf16_)
     sgs<__nv_bfloat16, float>(gs_vals16_.p, rdiag32_.p, x, y, s, false, sweep);
@@ -2450,12 +2459,7 @@ SolveResult KrylovSolver::mixed(const nw_solver_cfg& cfg, double tol,
   const int64_t n = A_.n;
   ensure_f32(s);
   gs_bf16_ = cfg.precision == NW_PREC_MIXED_BF16;
-  if (gs_bf16_ && gs_vals16_.n != gs_vals32_.n) {
-    gs_vals16_.resize(gs_vals32_.n);
-    if (gs_vals32_.n)
-      to_bf16_vals_k<<<grid1(int64_t(gs_vals32_.n)), kBlock, 0, s>>>(int64_t(gs_vals32_.n), gs_vals32_.p,
-                                                                    gs_vals16_.p);
-  }
+  if (gs_bf16_) ensure_bf16(s);
   const int m = std::min(m_, std::max(1, cfg.inner_kspace > 0 ? cfg.inner_kspace : cfg.kspace));
   const double itol = cfg.inner_tolerance > 0 ? cfg.inner_tolerance : 1e-4;
   SolveResult res;

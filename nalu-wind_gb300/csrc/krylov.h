@@ -110,6 +110,7 @@ class KrylovSolver {
   }
   bool has_learned() const { return net_ && cl_; }
   void ensure_f32(cudaStream_t s);
+  void ensure_bf16(cudaStream_t s);  // after ensure_f32
   // FP32 preconditioner application (Jacobi, SGS or learned) of the mixed
   // method; y and x must not alias.
   void precond32(const Precond& pc, const float* x, float* y, cudaStream_t s);
@@ -227,7 +228,7 @@ class KrylovSolver {
   // FP32 copies for the inner solve of the mixed method
   DeviceArray<float> vals32_, rdiag32_, V32_, w32_, z32_, r32_;
   int64_t ld32_ = 0;  // leading dimension of the FP32 basis (n rounded up to 32)
-  bool f32_valid_ = false;
+  bool f32_valid_ = false, bf16_valid_ = false;
   void mdot64(int nv, const double* V, int64_t ld, const double* w, double* out, double* acc, cudaStream_t s);
   void maxpy64(int nv, const double* V, int64_t ld, const double* h, double* w, double* nrm, cudaStream_t s,
                const GivensCol* gc = nullptr);
