@@ -36,6 +36,7 @@
 #include "krylov.h"
 #include "last_block.h"
 #include "learned.h"
+#include "pdl.h"
 
 namespace nw {
 namespace {
@@ -732,31 +733,34 @@ __global__ void __launch_bounds__(kBlock)
   const int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (k >= cnt) return;
   const int32_t i = rows[k];
+  const int64_t base = off[k >> 5] + (k & 31);
+  const int n = first ? 0 : len[k];
+  // batches of kGsBatch entries: every column and value load of the batch
+  // first, then every y gather, then the multiply-adds in column order
+  // (the same sum as one entry at a time, with the loads in flight
+  // together instead of one dependent pair per entry); the next batch's
+  // columns are loaded under the current one
+  int32_t c[kGsBatch];
+#pragma unroll
+  for (int j = 0; j < kGsBatch; ++j) c[j] = j < n ? cols[base + 32 * int64_t(j)] : i;
+  pdl_wait(v, rd, x, y);
   T s = x[i];
-  if (!first) {
-    const int64_t base = off[k >> 5] + (k & 31);
-    const int n = len[k];
-    // batches of kGsBatch entries: every column and value load of the batch
-    // first, then every y gather, then the multiply-adds in column order
-    // (the same sum as one entry at a time, with the loads in flight
-    // together instead of one dependent pair per entry)
-    for (int q = 0; q < n; q += kGsBatch) {
-      int32_t c[kGsBatch];
-      T a[kGsBatch], yv[kGsBatch];
+  const T r = rd[i];
+  for (int q = 0; q < n; q += kGsBatch) {
+    T a[kGsBatch], yv[kGsBatch];
 #pragma unroll
-      for (int j = 0; j < kGsBatch; ++j) {
-        const int64_t p = base + 32 * int64_t(q + j);
-        c[j] = q + j < n ? cols[p] : i;
-        a[j] = q + j < n ? T(v[p]) : T(0);
-      }
-#pragma unroll
-      for (int j = 0; j < kGsBatch; ++j) yv[j] = q + j < n ? y[c[j]] : T(0);
-#pragma unroll
-      for (int j = 0; j < kGsBatch; ++j)
-        if (q + j < n) s = fma(-a[j], yv[j], s);
+    for (int j = 0; j < kGsBatch; ++j) {
+      a[j] = q + j < n ? T(v[base + 32 * int64_t(q + j)]) : T(0);
+      yv[j] = q + j < n ? y[c[j]] : T(0);
     }
+#pragma unroll
+    for (int j = 0; j < kGsBatch; ++j)
+      c[j] = q + kGsBatch + j < n ? cols[base + 32 * int64_t(q + kGsBatch + j)] : i;
+#pragma unroll
+    for (int j = 0; j < kGsBatch; ++j)
+      if (q + j < n) s = fma(-a[j], yv[j], s);
   }
-  y[i] = s * rd[i];
+  y[i] = s * r;
 }
 
 // The dof classes of one colour of a system with `dof` rows a node: the rows
@@ -870,25 +874,30 @@ __global__ void __launch_bounds__(kBlock)
                const float* __restrict__ x, const float* __restrict__ y, float* __restrict__ r,
                int64_t zcnt, const int32_t* __restrict__ zrows) {
   const int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (k >= cnt) {
-    if (k - cnt < zcnt) r[zrows[k - cnt]] = 0.f;
+  const bool zero = k >= cnt;
+  if (zero && k - cnt >= zcnt) return;
+  const int32_t i = zero ? zrows[k - cnt] : rows[k];
+  const int64_t base = zero ? 0 : off[k >> 5] + (k & 31);
+  const int n = zero ? 0 : len[k];
+  int32_t c[kGsBatch];  // batched loads as in gs_sell_k
+#pragma unroll
+  for (int j = 0; j < kGsBatch; ++j) c[j] = j < n ? cols[base + 32 * int64_t(j)] : i;
+  pdl_wait(v, diag, x, y, r);
+  if (zero) {
+    r[i] = 0.f;
     return;
   }
-  const int32_t i = rows[k];
   float s = fmaf(-diag[i], y[i], x[i]);
-  const int64_t base = off[k >> 5] + (k & 31);
-  const int n = len[k];
-  for (int q = 0; q < n; q += kGsBatch) {  // batched loads as in gs_sell_k
-    int32_t c[kGsBatch];
+  for (int q = 0; q < n; q += kGsBatch) {
     float a[kGsBatch], yv[kGsBatch];
 #pragma unroll
     for (int j = 0; j < kGsBatch; ++j) {
-      const int64_t p = base + 32 * int64_t(q + j);
-      c[j] = q + j < n ? cols[p] : i;
-      a[j] = q + j < n ? v[p] : 0.f;
+      a[j] = q + j < n ? v[base + 32 * int64_t(q + j)] : 0.f;
+      yv[j] = q + j < n ? y[c[j]] : 0.f;
     }
 #pragma unroll
-    for (int j = 0; j < kGsBatch; ++j) yv[j] = q + j < n ? y[c[j]] : 0.f;
+    for (int j = 0; j < kGsBatch; ++j)
+      c[j] = q + kGsBatch + j < n ? cols[base + 32 * int64_t(q + kGsBatch + j)] : i;
 #pragma unroll
     for (int j = 0; j < kGsBatch; ++j)
       if (q + j < n) s = fmaf(-a[j], yv[j], s);
@@ -1028,13 +1037,15 @@ __global__ void __launch_bounds__(kBlock)
                const int64_t* __restrict__ dpos, const T* __restrict__ x, T* __restrict__ y) {
   const int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (k >= cnt) return;
-  const int64_t i = rows[k];
+  const int64_t i = rows[k], p1 = rp[i + 1], dp = dpos[i];
+  int64_t p = rp[i];
+  pdl_wait(v, x, y);
   T s = x[i];
-  for (int64_t p = rp[i]; p < rp[i + 1]; ++p) {
+  for (; p < p1; ++p) {
     const int64_t c = ci[p];
     if (c != i) s = rn_sub(s, rn_mul(T(v[p]), y[c]));
   }
-  y[i] = rn_div(s, T(v[dpos[i]]));
+  y[i] = rn_div(s, T(v[dp]));
 }
 
 // ILU(0) factorization of the rows of one forward level (IKJ order, Saad,
@@ -1075,15 +1086,17 @@ __global__ void __launch_bounds__(kBlock)
                        const T* __restrict__ lu, const T* __restrict__ x, T* __restrict__ y) {
   const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (t >= cnt) return;
-  const int64_t i = rows[t];
+  const int64_t i = rows[t], dp = dpos[i], pend = UPPER ? rp[i + 1] : dp;
+  int64_t p = UPPER ? dp + 1 : rp[i];
+  pdl_wait(lu, x, y);
   if (!UPPER) {
     T s = x[i];
-    for (int64_t p = rp[i]; p < dpos[i]; ++p) s = rn_sub(s, rn_mul(lu[p], y[ci[p]]));
+    for (; p < pend; ++p) s = rn_sub(s, rn_mul(lu[p], y[ci[p]]));
     y[i] = s;
   } else {
     T s = y[i];
-    for (int64_t p = dpos[i] + 1; p < rp[i + 1]; ++p) s = rn_sub(s, rn_mul(lu[p], y[ci[p]]));
-    y[i] = rn_div(s, lu[dpos[i]]);
+    for (; p < pend; ++p) s = rn_sub(s, rn_mul(lu[p], y[ci[p]]));
+    y[i] = rn_div(s, lu[dp]);
   }
 }
 
@@ -1531,7 +1544,7 @@ void KrylovSolver::sgs(const VT* vals, const T* rd, const T* x, T* y, cudaStream
   auto pass = [&](int c, int first) {
     const int64_t b = gs_cptr_[c], cnt = gs_cptr_[c + 1] - b;
     if (cnt)
-      gs_sell_k<VT, T><<<grid1(cnt), kBlock, 0, s>>>(cnt, gs_rows_.p + b, gs_off_.p + gs_slice0_[c],
+      pdl_launch(gs_sell_k<VT, T>, grid1(cnt), kBlock, 0, s, cnt, gs_rows_.p + b, gs_off_.p + gs_slice0_[c],
                                                      gs_len_.p + b, gs_cols_.p, vals, rd, x, y,
                                                      first);
   };
@@ -1557,7 +1570,7 @@ void KrylovSolver::sgs_residual32(const float* x, const float* y, float* r, cuda
     if (c == last && nc > 1) continue;
     const int64_t b = gs_cptr_[c], cnt = c == last ? 0 : gs_cptr_[c + 1] - b;
     if (cnt + zcnt)
-      gs_resid_k<<<grid1(cnt + zcnt), kBlock, 0, s>>>(cnt, gs_rows_.p + b, gs_off_.p + gs_slice0_[c],
+      pdl_launch(gs_resid_k, grid1(cnt + zcnt), kBlock, 0, s, cnt, gs_rows_.p + b, gs_off_.p + gs_slice0_[c],
                                                       gs_len_.p + b, gs_cols_.p, gs_vals32_.p, diag32_.p,
                                                       x, y, r, zcnt, zrows);
     zcnt = 0;
@@ -1738,7 +1751,7 @@ void KrylovSolver::sgs_natural(const VT* vals, const T* x, T* y, cudaStream_t s)
     for (size_t l = 0; l + 1 < ptr.size(); ++l) {
       const int64_t cnt = ptr[l + 1] - ptr[l];
       if (cnt)
-        gs_level_k<VT, T><<<grid1(cnt), kBlock, 0, s>>>(cnt, rows + ptr[l], A_.row_ptr, A_.col_idx, vals,
+        pdl_launch(gs_level_k<VT, T>, grid1(cnt), kBlock, 0, s, cnt, rows + ptr[l], A_.row_ptr, A_.col_idx, vals,
                                                          dpos_.p, x, y);
     }
   }
@@ -1767,13 +1780,13 @@ void KrylovSolver::ilu0_solve(const T* lu, const T* x, T* y, cudaStream_t s) {
   for (size_t l = 0; l + 1 < fl_ptr_.size(); ++l) {
     const int64_t cnt = fl_ptr_[l + 1] - fl_ptr_[l];
     if (cnt)
-      ilu0_solve_level_k<false, T><<<grid1(cnt), kBlock, 0, s>>>(cnt, fl_rows_.p + fl_ptr_[l], A_.row_ptr,
+      pdl_launch(ilu0_solve_level_k<false, T>, grid1(cnt), kBlock, 0, s, cnt, fl_rows_.p + fl_ptr_[l], A_.row_ptr,
                                                                   A_.col_idx, dpos_.p, lu, x, y);
   }
   for (size_t l = 0; l + 1 < bl_ptr_.size(); ++l) {
     const int64_t cnt = bl_ptr_[l + 1] - bl_ptr_[l];
     if (cnt)
-      ilu0_solve_level_k<true, T><<<grid1(cnt), kBlock, 0, s>>>(cnt, bl_rows_.p + bl_ptr_[l], A_.row_ptr,
+      pdl_launch(ilu0_solve_level_k<true, T>, grid1(cnt), kBlock, 0, s, cnt, bl_rows_.p + bl_ptr_[l], A_.row_ptr,
                                                                  A_.col_idx, dpos_.p, lu, y, y);
   }
   NW_CUDA(cudaGetLastError());

@@ -24,6 +24,7 @@
 
 #include "last_block.h"
 #include "learned.h"
+#include "pdl.h"
 
 namespace nw {
 namespace {
@@ -239,6 +240,7 @@ __global__ void __launch_bounds__(kB)
   if (I >= nc) return;
   float a0 = 0.f, a1 = 0.f;
   const int64_t dpos = cdiag[I], q1 = cptr[I + 1];
+  pdl_wait(wgt, xc);
   for (int64_t q = cptr[I]; q < q1; q += 32) {
     const bool on = q + lane < q1 && q + lane != dpos;
     const int32_t c = on ? ccol[q + lane] : -1;
@@ -336,6 +338,7 @@ __device__ __forceinline__ void block_sum(int nblocks, double (&v)[W], F part) {
 __global__ void __launch_bounds__(kB)
     input_k(int64_t nc, const float* __restrict__ rc, const float* __restrict__ dinv, float* __restrict__ u,
             float* partial, float* __restrict__ scal, int* __restrict__ ticket) {
+  pdl_wait(rc, dinv, u, partial, scal, ticket);
   __shared__ float red[kB / 32];
   const int64_t I = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   float v = 0.f;
@@ -373,6 +376,7 @@ __global__ void __launch_bounds__(kB)
   const int64_t I = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (I >= nc) return;
+  pdl_wait(wgt, u, scal, w0, x, ax, xc);
   const float inv = scal[1];
   const float xi = u[I] * inv;
   float a = 0.f;
@@ -397,6 +401,7 @@ __global__ void __launch_bounds__(kB)
   const int64_t I = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (I >= nc) return;
+  pdl_wait(h3, wout, scal, y, ec);
   const uint32_t v = *reinterpret_cast<const uint32_t*>(h3 + I * 64 + 2 * lane);
   float s = bf2f(uint16_t(v & 0xffffu)) * wout[2 * lane] + bf2f(uint16_t(v >> 16)) * wout[2 * lane + 1];
   for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
@@ -414,6 +419,7 @@ __global__ void coarse_jacobi_k(int64_t nc, const int64_t* __restrict__ cptr,
                                 const float* __restrict__ wgt, const float* __restrict__ dinv,
                                 const float* __restrict__ rc, const float* __restrict__ ein,
                                 float* __restrict__ eout) {
+  pdl_wait(wgt, dinv, rc, ein, eout);
   const int64_t I = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (I >= nc) return;
   float v = dinv[I] * rc[I];
@@ -447,6 +453,7 @@ __global__ void __launch_bounds__(kRowLanes * kRowBlock)
                    const float* __restrict__ ec, const float* __restrict__ rc,
                    float* __restrict__ aec, float* partial, float* __restrict__ scal,
                    int* __restrict__ ticket) {
+  pdl_wait(wgt, dinv, ec, rc, aec, partial, scal, ticket);
   __shared__ float red[2][kRowBlock];
   const int row = threadIdx.x / kRowLanes, sub = threadIdx.x % kRowLanes;
   const int64_t I = int64_t(blockIdx.x) * kRowBlock + row;
@@ -649,8 +656,10 @@ __global__ void __launch_bounds__(kB)
   const int64_t I = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (I >= nc) return;
+  const int64_t k0 = mptr[I], k1 = mptr[I + 1];
+  pdl_wait(r, rc);
   float s = 0.f;
-  for (int64_t k = mptr[I] + lane; k < mptr[I + 1]; k += 32) s += r[mrows[k]];
+  for (int64_t k = k0 + lane; k < k1; k += 32) s += r[mrows[k]];
   for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
   if (lane == 0) rc[I] = s;
 }
@@ -660,7 +669,10 @@ __global__ void prolong_add_k(int64_t nf, const int32_t* __restrict__ agg,
                               const float* __restrict__ ec, const float* __restrict__ alpha,
                               float* __restrict__ z) {
   const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i < nf) z[i] += *alpha * ec[agg[i]];
+  if (i >= nf) return;
+  const int32_t I = agg[i];
+  pdl_wait(ec, alpha, z);
+  z[i] += *alpha * ec[I];
 }
 
 uint64_t fnv1a(const void* data, size_t n) {
@@ -701,11 +713,11 @@ void launch_gemm_wgrad_tc(const uint16_t* xc, const uint16_t* dz, float* partial
 }
 
 void launch_restrict(const CoarseLevel& cl, const float* r, float* rc, cudaStream_t s) {
-  restrict_k<<<gridn(cl.nc * 32), kB, 0, s>>>(cl.nc, cl.mptr.p, cl.mrows.p, r, rc);
+  pdl_launch(restrict_k, gridn(cl.nc * 32), kB, 0, s, cl.nc, cl.mptr.p, cl.mrows.p, r, rc);
 }
 void launch_prolong_add(const CoarseLevel& cl, const float* ec, const float* alpha, float* z,
                         cudaStream_t s) {
-  prolong_add_k<<<gridn(cl.nf), kB, 0, s>>>(cl.nf, cl.agg.p, ec, alpha, z);
+  pdl_launch(prolong_add_k, gridn(cl.nf), kB, 0, s, cl.nf, cl.agg.p, ec, alpha, z);
 }
 
 // ---------------------------------------------------------------------------
@@ -1031,16 +1043,16 @@ void LearnedNet::forward(const CoarseLevel& cl, const float* wgt, const float* d
   const int64_t nc = cl.nc;
   work.resize(nc, s);
   const unsigned gw = gridn(nc * 32);  // warp per row
-  input_k<<<gridn(nc), kB, 0, s>>>(nc, rc, dinv, work.u.p, work.partial.p, work.scal.p, work.ticket.p);
-  layer0_k<<<gw, kB, 0, s>>>(nc, cl.cptr.p, cl.ccol.p, cl.cdiag.p, wgt, work.u.p, work.scal.p,
+  pdl_launch(input_k, gridn(nc), kB, 0, s, nc, rc, dinv, work.u.p, work.partial.p, work.scal.p, work.ticket.p);
+  pdl_launch(layer0_k, gw, kB, 0, s, nc, cl.cptr.p, cl.ccol.p, cl.cdiag.p, wgt, work.u.p, work.scal.p,
                              params.p + kOffW0, work.x.p, work.ax.p, work.xc1.p);
   uint16_t* xcs[4] = {work.xc1.p, work.xc2.p, work.xc3.p, nullptr};
   for (int l = 0; l < 3; ++l) {
-    agg_fwd_k<<<gw, kB, 0, s>>>(nc, cl.cptr.p, cl.ccol.p, cl.cdiag.p, wgt, xcs[l]);
+    pdl_launch(agg_fwd_k, gw, kB, 0, s, nc, cl.cptr.p, cl.ccol.p, cl.cdiag.p, wgt, xcs[l]);
     uint16_t* out = l < 2 ? xcs[l + 1] : work.h3.p;
     launch_gemm_fwd_tma(xcs[l], wtbf.p + size_t(l) * kIn2 * kHid, out, nc, l < 2 ? 128 : 64, s);
   }
-  output_k<<<gw, kB, 0, s>>>(nc, work.h3.p, params.p + kOffWout, work.scal.p, work.y.p, ec);
+  pdl_launch(output_k, gw, kB, 0, s, nc, work.h3.p, params.p + kOffWout, work.scal.p, work.y.p, ec);
   NW_CUDA(cudaGetLastError());
 }
 
@@ -1051,13 +1063,13 @@ void LearnedNet::coarse_correction(const CoarseLevel& cl, const float* rc, float
     forward(cl, cl.wgt.p, cl.dinv.p, rc, ec, s);
   } else {
     work.resize(cl.nc, s);
-    coarse_jacobi_k<<<nb, kB, 0, s>>>(cl.nc, cl.cptr.p, cl.ccol.p, cl.cdiag.p, cl.wgt.p, cl.dinv.p, rc,
+    pdl_launch(coarse_jacobi_k, nb, kB, 0, s, cl.nc, cl.cptr.p, cl.ccol.p, cl.cdiag.p, cl.wgt.p, cl.dinv.p, rc,
                                       nullptr, coarse_mode == 1 ? ec : work.u.p);
     if (coarse_mode == 2)
-      coarse_jacobi_k<<<nb, kB, 0, s>>>(cl.nc, cl.cptr.p, cl.ccol.p, cl.cdiag.p, cl.wgt.p, cl.dinv.p, rc,
+      pdl_launch(coarse_jacobi_k, nb, kB, 0, s, cl.nc, cl.cptr.p, cl.ccol.p, cl.cdiag.p, cl.wgt.p, cl.dinv.p, rc,
                                         work.u.p, ec);
   }
-  coarse_apply_k<<<gridn(cl.nc, kRowBlock), kB, 0, s>>>(cl.nc, cl.cptr.p, cl.ccol.p, cl.cdiag.p, cl.wgt.p, cl.dinv.p,
+  pdl_launch(coarse_apply_k, gridn(cl.nc, kRowBlock), kB, 0, s, cl.nc, cl.cptr.p, cl.ccol.p, cl.cdiag.p, cl.wgt.p, cl.dinv.p,
                                    ec, rc, work.aec.p, work.partial.p, work.scal.p, work.ticket.p);
   NW_CUDA(cudaGetLastError());
 }
@@ -1071,7 +1083,7 @@ double LearnedNet::forward_backward(const CoarseLevel& cl, const float* wgt,
   forward(cl, wgt, dinv, rc, ec, s);
   const unsigned gw = gridn(nc * 32);
   const int nb = int(gridn(nc));
-  coarse_apply_k<<<gridn(nc, kRowBlock), kB, 0, s>>>(nc, cl.cptr.p, cl.ccol.p, cl.cdiag.p, wgt, dinv, ec, rc,
+  pdl_launch(coarse_apply_k, gridn(nc, kRowBlock), kB, 0, s, nc, cl.cptr.p, cl.ccol.p, cl.cdiag.p, wgt, dinv, ec, rc,
                                    work.aec.p, work.partial.p, work.scal.p, work.ticket.p);
   float sc[4];
   NW_CUDA(cudaMemcpyAsync(sc, work.scal.p, sizeof(sc), cudaMemcpyDeviceToHost, s));

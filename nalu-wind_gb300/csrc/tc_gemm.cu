@@ -21,6 +21,7 @@
 #include <cstdint>
 
 #include "nw_internal.h"
+#include "pdl.h"
 
 namespace nw {
 namespace {
@@ -290,6 +291,9 @@ __global__ void __launch_bounds__(128)
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bars + i)) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  pdl_wait(out);
+  if (tid == 0) {
     expect_tx(wbar, 2 * kPanelB);
     tma_load_2d(b0, &map_w, 0, 0, wbar);
     tma_load_2d(b0 + kPanelB, &map_w, 64, 0, wbar);
@@ -777,7 +781,7 @@ void launch_gemm_fwd_tma(const uint16_t* a, const uint16_t* wt, uint16_t* out, i
   const CUtensorMap mw = make_map(wt, kN, kN);
   const int64_t tiles = (m + kTileM - 1) / kTileM;
   const unsigned grid = unsigned(tiles < ctas ? tiles : ctas);
-  gemm_fwd_tma_k<<<grid, 128, kSmemTma, s>>>(ma, mw, out, m, ldo);
+  pdl_launch(gemm_fwd_tma_k, grid, 128, kSmemTma, s, ma, mw, out, m, ldo);
   NW_CUDA(cudaGetLastError());
 }
 
