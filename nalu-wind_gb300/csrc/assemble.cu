@@ -964,7 +964,7 @@ __global__ void __launch_bounds__(kThreads)
   if (k >= n) return;
   const int64_t node = nodes[k];
   if (node < 0 || node >= num_nodes) {
-    atomicExch(err, 1);
+    *err = 1;
     return;
   }
   if (end <= begin) return;

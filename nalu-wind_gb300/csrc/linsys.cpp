@@ -11,6 +11,7 @@
 #include <new>
 #include <numeric>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "assemble.h"
@@ -77,7 +78,7 @@ struct nw_linsys {
   DeviceArray<int32_t> f_items, f_in_ptr, f_in, f_out_ptr, f_out;
   DeviceArray<int> f_eflag, f_rflag, f_ticket, f_err;
   DeviceArray<double> ring;
-  DeviceArray<int> err;
+  int* err = nullptr;  // pinned: a bad node index of a row reset, zero between calls
   DeviceArray<int64_t> scratch_lid;
   DeviceArray<double> scratch_vals;
   KrylovSolver solver;
@@ -230,6 +231,7 @@ nw_status nw_linsys_destroy(nw_linsys* ls) {
     if (ls->solve_in) cudaEventDestroy(ls->solve_in);
     if (ls->solve_out) cudaEventDestroy(ls->solve_out);
     if (ls->solve_stream) cudaStreamDestroy(ls->solve_stream);
+    if (ls->err) cudaFreeHost(ls->err);
     delete ls;
   });
 }
@@ -364,8 +366,8 @@ nw_status nw_linsys_finalize(nw_linsys* ls) {
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0)
       fail(NW_NO_DEVICE, "no CUDA device");
     NW_CUDA(cudaSetDevice(ls->device));
-    ls->err.resize(1);
-    NW_CUDA(cudaMemset(ls->err.p, 0, sizeof(int)));
+    if (!ls->err) NW_CUDA(cudaMallocHost(&ls->err, sizeof(int)));
+    *ls->err = 0;
     HostGraph& g = ls->g;
     cudaStream_t s = ls->stream;
     ls->row_ptr.upload(g.row_ptr, s);
@@ -737,15 +739,12 @@ nw_status nw_linsys_apply_dirichlet(nw_linsys* ls, int64_t n,
         end > ls->num_dof || begin > end)
       fail(NW_INVALID_ARG, "bad Dirichlet arguments");
     materialize_zero(ls);
-    NW_CUDA(cudaMemsetAsync(ls->err.p, 0, sizeof(int), ls->stream));
     launch_reset_rows(ls->stream, n, nodes, ls->node_lid.p, ls->num_dof, begin,
                       end, ls->row_ptr.p, ls->col_idx.p, ls->values.p,
-                      ls->rhs.p, 1.0, 0.0, q, bc, ls->g.num_nodes, ls->err.p);
+                      ls->rhs.p, 1.0, 0.0, q, bc, ls->g.num_nodes, ls->err);
     NW_CUDA(cudaGetLastError());
-    int herr = 0;
-    NW_CUDA(cudaMemcpyAsync(&herr, ls->err.p, sizeof(int), cudaMemcpyDeviceToHost, ls->stream));
     NW_CUDA(cudaStreamSynchronize(ls->stream));
-    if (herr) fail(NW_INVALID_ARG, "Dirichlet node index out of range");
+    if (std::exchange(*ls->err, 0)) fail(NW_INVALID_ARG, "Dirichlet node index out of range");
   });
 }
 
@@ -758,16 +757,13 @@ nw_status nw_linsys_reset_rows(nw_linsys* ls, int64_t n, const int64_t* nodes,
         begin > end)
       fail(NW_INVALID_ARG, "bad resetRows arguments");
     materialize_zero(ls);
-    NW_CUDA(cudaMemsetAsync(ls->err.p, 0, sizeof(int), ls->stream));
     launch_reset_rows(ls->stream, n, nodes, ls->node_lid.p, ls->num_dof, begin,
                       end, ls->row_ptr.p, ls->col_idx.p, ls->values.p,
                       ls->rhs.p, diag_value, rhs_residual, nullptr, nullptr,
-                      ls->g.num_nodes, ls->err.p);
+                      ls->g.num_nodes, ls->err);
     NW_CUDA(cudaGetLastError());
-    int herr = 0;
-    NW_CUDA(cudaMemcpyAsync(&herr, ls->err.p, sizeof(int), cudaMemcpyDeviceToHost, ls->stream));
     NW_CUDA(cudaStreamSynchronize(ls->stream));
-    if (herr) fail(NW_INVALID_ARG, "resetRows node index out of range");
+    if (std::exchange(*ls->err, 0)) fail(NW_INVALID_ARG, "resetRows node index out of range");
   });
 }
 
