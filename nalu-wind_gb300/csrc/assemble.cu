@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(kThreads)
 // spread the FP64 work evenly over the SMs: 346 -> 338 us on 476,280 nodes with
 // limiter and tanh (blocks of 256 and 64).
 constexpr int kScalarBlock = 64;
-template <bool LIMITER, bool TANH, bool ALPHA>
+template <bool LIMITER, bool TANH, bool ALPHA, bool NODE>
 __global__ void __launch_bounds__(kScalarBlock)
     scalar_edge_k(int64_t E, const int2* __restrict__ edges, const double* __restrict__ coords,
                   const double* __restrict__ vrtm, const double* __restrict__ q, const double* __restrict__ dqdx,
@@ -148,7 +148,10 @@ __global__ void __launch_bounds__(kScalarBlock)
   }
   const double w = asq * fast_rcp(axdx);
   const double visc = 0.5 * (dflux[L] + dflux[R]);
-  const double den = fma(0.5, dor[L] + dor[R], eps);
+  // mu / rho: from the node pre-pass, or (small systems) here from rho
+  const double dsum = NODE ? dor[L] + dor[R]
+                           : __dadd_rn(__dmul_rn(dflux[L], fast_rcp(dor[L])), __dmul_rn(dflux[R], fast_rcp(dor[R])));
+  const double den = fma(0.5, dsum, eps);
   double pec;
   if (TANH) {
     const double pe = (0.5 * fabs(udx)) * fast_rcp(den);
@@ -258,14 +261,17 @@ __global__ void __launch_bounds__(kThreads)
       ldd(Gpdx + 3 * n + 2) * iu, ldd(pressure + n));
 }
 
-template <bool PLAIN>
-__global__ void __launch_bounds__(kThreads, 6)
+struct ContinuityNodeFields {
+  const double *velocity, *Gpdx, *density, *udiag;
+};
+template <bool PLAIN, bool NODE>
+__global__ void __launch_bounds__(kThreads, NODE ? 6 : 4)
     continuity_edge_fast_k(int64_t E, const int2* __restrict__ edges,
                            const double* __restrict__ coords,
                            const dd* __restrict__ nodebuf,
                            const double* __restrict__ pressure,
                            const double* __restrict__ area, dd noc,
-                           dd inv_tau, dd* __restrict__ buf) {
+                           dd inv_tau, dd* __restrict__ buf, ContinuityNodeFields nf) {
   const int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (e >= E) return;
   const int2 lr = edges[e];
@@ -273,7 +279,16 @@ __global__ void __launch_bounds__(kThreads, 6)
   // sums over the two nodes; a record is two 32-byte loads (four 16-byte
   // loads cost twice the L1 lookups)
   dd n[7];
-  {
+  if constexpr (!NODE) {  // the two records formed here
+    const dd iul = dd_rcp(ldd(nf.udiag + L)), iur = dd_rcp(ldd(nf.udiag + R));
+    const dd rl = ldd(nf.density + L), rr = ldd(nf.density + R);
+    n[0] = iul + iur;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      n[1 + d] = rl * ldd(nf.velocity + 3 * L + d) + rr * ldd(nf.velocity + 3 * R + d);
+      n[4 + d] = ldd(nf.Gpdx + 3 * L + d) * iul + ldd(nf.Gpdx + 3 * R + d) * iur;
+    }
+  } else {
     double a[4], b[4];
     const double* pl = reinterpret_cast<const double*>(nodebuf + kNodeStride * L);
     const double* pr = reinterpret_cast<const double*>(nodebuf + kNodeStride * R);
@@ -1038,23 +1053,36 @@ void launch_scalar_edges(cudaStream_t s, int64_t E, int64_t N, const int2* edges
                          const nw_scalar_fields& f, const ScalarOpts& o,
                          double* buf, double* nodebuf) {
   if (E == 0) return;
-  scalar_node_k<<<grid_for(N), kThreads, 0, s>>>(N, f.density, f.diff_coeff, nodebuf);
+  // Small systems skip the node pre-pass: its launch costs more than the two
+  // reciprocals an edge it saves. Pass with and without it, default options:
+  // 104 k edges 44.0 and 42.6 us, 267 k edges 72.5 and 73.3, 799 k 153 and 163
+  const bool node = E > 131072;
+  if (node) scalar_node_k<<<grid_for(N), kThreads, 0, s>>>(N, f.density, f.diff_coeff, nodebuf);
   const ScalarArgs a{o.alpha, o.alpha_upw, 1.0 - o.alpha, 1.0 - o.alpha_upw, o.upw_factor,
                      0.5 * o.hybrid_factor, o.tanh_trans, -2.0 / o.tanh_width};
   auto go = [&](auto kernel) {
-    kernel<<<grid_for(E, kScalarBlock), kScalarBlock, 0, s>>>(E, edges, f.coords, f.velocity_rtm, f.q, f.dqdx, f.diff_coeff, nodebuf,
-                                            f.area, f.mdot, a, buf);
+    kernel<<<grid_for(E, kScalarBlock), kScalarBlock, 0, s>>>(E, edges, f.coords, f.velocity_rtm, f.q, f.dqdx,
+                                                              f.diff_coeff, node ? nodebuf : f.density, f.area,
+                                                              f.mdot, a, buf);
   };
-  const int which = (o.use_limiter ? 4 : 0) + (o.tanh_form ? 2 : 0) + (o.alpha != 0.0 ? 1 : 0);
+  const int which = (o.use_limiter ? 8 : 0) + (o.tanh_form ? 4 : 0) + (o.alpha != 0.0 ? 2 : 0) + (node ? 1 : 0);
   switch (which) {
-    case 0: go(scalar_edge_k<false, false, false>); break;
-    case 1: go(scalar_edge_k<false, false, true>); break;
-    case 2: go(scalar_edge_k<false, true, false>); break;
-    case 3: go(scalar_edge_k<false, true, true>); break;
-    case 4: go(scalar_edge_k<true, false, false>); break;
-    case 5: go(scalar_edge_k<true, false, true>); break;
-    case 6: go(scalar_edge_k<true, true, false>); break;
-    default: go(scalar_edge_k<true, true, true>); break;
+    case 0: go(scalar_edge_k<false, false, false, false>); break;
+    case 1: go(scalar_edge_k<false, false, false, true>); break;
+    case 2: go(scalar_edge_k<false, false, true, false>); break;
+    case 3: go(scalar_edge_k<false, false, true, true>); break;
+    case 4: go(scalar_edge_k<false, true, false, false>); break;
+    case 5: go(scalar_edge_k<false, true, false, true>); break;
+    case 6: go(scalar_edge_k<false, true, true, false>); break;
+    case 7: go(scalar_edge_k<false, true, true, true>); break;
+    case 8: go(scalar_edge_k<true, false, false, false>); break;
+    case 9: go(scalar_edge_k<true, false, false, true>); break;
+    case 10: go(scalar_edge_k<true, false, true, false>); break;
+    case 11: go(scalar_edge_k<true, false, true, true>); break;
+    case 12: go(scalar_edge_k<true, true, false, false>); break;
+    case 13: go(scalar_edge_k<true, true, false, true>); break;
+    case 14: go(scalar_edge_k<true, true, true, false>); break;
+    default: go(scalar_edge_k<true, true, true, true>); break;
   }
 }
 
@@ -1066,7 +1094,7 @@ dd dd_param(double x) { return dd_from_double(x); }
 
 void launch_continuity_edge_range(cudaStream_t s, int64_t n0, int64_t n1, int64_t e0, int64_t e1,
                                   const int2* edges, const nw_continuity_fields& f,
-                                  const ContinuityOpts& o, double* buf, double* nodebuf) {
+                                  const ContinuityOpts& o, double* buf, double* nodebuf, bool node) {
   // the edge kernels index edges, area vectors and records from 0: shift
   // the per-edge pointers to the range
   const int64_t n = e1 > e0 ? e1 - e0 : 0;
@@ -1075,18 +1103,20 @@ void launch_continuity_edge_range(cudaStream_t s, int64_t n0, int64_t n1, int64_
   const double* ar = f.area + 3 * e0;
   if (nodebuf && continuity_fast_path(o)) {
     dd* nb = reinterpret_cast<dd*>(nodebuf);
-    if (n1 > n0)
+    if (node && n1 > n0)
       continuity_node_k<<<grid_for(n1 - n0), kThreads, 0, s>>>(
           n0, n1, f.velocity, f.dpdx, f.density, f.pressure, f.udiag, nb);
     if (n) {
       auto go = [&](auto kernel) {
         kernel<<<grid_for(n), kThreads, 0, s>>>(n, er, f.coords, nb, f.pressure, ar, dd_param(o.noc_fac),
-                                                dd_param(1.0 / o.tau_scale), b);
+                                                dd_param(1.0 / o.tau_scale), b,
+                                                ContinuityNodeFields{f.velocity, f.dpdx, f.density, f.udiag});
       };
-      if (o.noc_fac == 1.0)
-        go(continuity_edge_fast_k<true>);
+      const bool plain = o.noc_fac == 1.0;
+      if (node)
+        plain ? go(continuity_edge_fast_k<true, true>) : go(continuity_edge_fast_k<false, true>);
       else
-        go(continuity_edge_fast_k<false>);
+        plain ? go(continuity_edge_fast_k<true, false>) : go(continuity_edge_fast_k<false, false>);
     }
   } else if (n) {
     ContinuityDD c;
@@ -1107,7 +1137,11 @@ void launch_continuity_edges(cudaStream_t s, int64_t E, int64_t N,
                              const ContinuityOpts& o, double* buf,
                              double* nodebuf) {
   if (E == 0) return;
-  launch_continuity_edge_range(s, 0, N, 0, E, edges, f, o, buf, nodebuf);
+  // Small systems form the node records in the edge kernel (the same
+  // operations): a launch costs more than the repeated ones. With and without
+  // the pre-pass: 19 k edges 21.2 and 17.9 us, 267 k 32.5 and 30.0. Ranges keep
+  // the pre-pass, whose records later ranges read.
+  launch_continuity_edge_range(s, 0, N, 0, E, edges, f, o, buf, nodebuf, E > 262144);
 }
 
 void launch_continuity_edges(cudaStream_t s, int64_t E, const int2* edges,
