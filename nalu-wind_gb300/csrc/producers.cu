@@ -32,9 +32,13 @@ __device__ __forceinline__ dd ldd(const double* p) { return dd_from_double(*p); 
 //
 // Bound by instruction issue: products stay in float pairs, but sums of FP64
 // inputs and rho u are formed in FP64 (ten operations an edge on the
-// otherwise idle pipe), each split once. PLAIN: noc = interp = 1.
+// otherwise idle pipe), each split once. PLAIN: noc = interp = 1. It also waits
+// for the gathers of two random nodes: twelve blocks of 128 (40 registers) took
+// the four producers on 1,167,183 edges of tets from 144 us (four of 256) to
+// 137.6; ten 138.2, fourteen 141.6.
+constexpr int kMdotBlock = 128;
 template <bool PLAIN>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kMdotBlock, 12)
     mdot_k(int64_t E, const int2* __restrict__ edges, const double* __restrict__ coords,
            const double* __restrict__ velocity, const double* __restrict__ Gpdx,
            const double* __restrict__ density, const double* __restrict__ pressure,
@@ -92,7 +96,7 @@ __device__ __forceinline__ void dd_mac(dd& acc, dd a, dd b) {
 // (incidence, edge, nodal values), hidden by many warps: 40 a SM or more
 // measured better than two to four edges loaded together at fewer. 172,032
 // nodes and 1,167,183 edges of tets: 68 -> 43 us (vector), 38 -> 25 (scalar);
-// mdot above 58 -> 39, the Peclet factor below 28 -> 23, all with smaller
+// mdot above 58 -> 36, the Peclet factor below 28 -> 23, all with smaller
 // errors against 64 bits (splits to the nearest pair).
 template <int DIM1>
 __global__ void __launch_bounds__(DIM1 == 3 ? 128 : kThreads, DIM1 == 3 ? 10 : 6)
@@ -220,7 +224,7 @@ extern "C" nw_status nw_compute_mdot_edges(nw_linsys* ls, const nw_continuity_fi
       nw::fail(NW_INVALID_ARG, "null field pointer");
     if (v.num_edges == 0) return;
     auto go = [&](auto kernel) {
-      kernel<<<nw::grid_for(v.num_edges), nw::kThreads, 0, v.stream>>>(
+      kernel<<<unsigned((v.num_edges + nw::kMdotBlock - 1) / nw::kMdotBlock), nw::kMdotBlock, 0, v.stream>>>(
           v.num_edges, v.edges, f->coords, f->velocity, f->dpdx, f->density, f->pressure, f->udiag, f->area,
           dd_from_double(noc_fac), dd_from_double(1.0 - noc_fac), interp_together, 1.0 - interp_together, mdot);
     };
