@@ -230,9 +230,10 @@ __global__ void __launch_bounds__(kScalarBlock)
 // The edge phase is bound by its 580 instructions an edge (56 % of the issue
 // slots) and the latency of two random records: 88 us on 128x128x64 hexes with
 // 16-byte record loads and 4 resident blocks a SM. Records read as 32-byte
-// loads and summed on arrival leave 40 registers and six blocks: the whole
-// assembly takes 147 us, 159 before (4 blocks 158, 5 blocks 150). PLAIN: the
-// default noc = 1 needs no product with it.
+// loads and summed on arrival leave 40 registers, 1,536 threads a SM in blocks
+// of 128: the whole assembly takes 145 us, 159 before (blocks of 256: four 158,
+// five 150, six 147; blocks of 64 147; 32 registers 148.5). PLAIN: the default
+// noc = 1 needs no product with it.
 constexpr int kNodeStride = 8;  // dd slots (8 bytes each) per node
 
 __device__ __forceinline__ dd ldd(const double* p) { return dd_from_double(*p); }
@@ -261,11 +262,12 @@ __global__ void __launch_bounds__(kThreads)
       ldd(Gpdx + 3 * n + 2) * iu, ldd(pressure + n));
 }
 
+constexpr int kContinuityBlock = 128;
 struct ContinuityNodeFields {
   const double *velocity, *Gpdx, *density, *udiag;
 };
 template <bool PLAIN, bool NODE>
-__global__ void __launch_bounds__(kThreads, NODE ? 6 : 4)
+__global__ void __launch_bounds__(kContinuityBlock, NODE ? 12 : 8)
     continuity_edge_fast_k(int64_t E, const int2* __restrict__ edges,
                            const double* __restrict__ coords,
                            const dd* __restrict__ nodebuf,
@@ -1108,7 +1110,7 @@ void launch_continuity_edge_range(cudaStream_t s, int64_t n0, int64_t n1, int64_
           n0, n1, f.velocity, f.dpdx, f.density, f.pressure, f.udiag, nb);
     if (n) {
       auto go = [&](auto kernel) {
-        kernel<<<grid_for(n), kThreads, 0, s>>>(n, er, f.coords, nb, f.pressure, ar, dd_param(o.noc_fac),
+        kernel<<<grid_for(n, kContinuityBlock), kContinuityBlock, 0, s>>>(n, er, f.coords, nb, f.pressure, ar, dd_param(o.noc_fac),
                                                 dd_param(1.0 / o.tau_scale), b,
                                                 ContinuityNodeFields{f.velocity, f.dpdx, f.density, f.udiag});
       };
