@@ -47,7 +47,7 @@ double warp_tree(double* a) {
   return a[0];
 }
 
-// reduce_partials_k: thread t sums partials t, t + 256, ...; then a shared
+// final sums of a reduction: thread t sums partials t, t + 256, ...; then a shared
 // memory tree
 double reduce_partials(const double* p, int64_t G) {
   double sh[kBlock];
@@ -62,7 +62,7 @@ double reduce_partials(const double* p, int64_t G) {
 }
 
 // warp sums of per-thread values, then thread-serial sum over the block's
-// warps (the block stage of mdot_k / maxpy_k)
+// warps (the block stage of mdot64_k / maxpy64_k)
 double block_sum(const double* thread_vals) {
   double red[kWarps];
   for (int w = 0; w < kWarps; ++w) {
@@ -75,7 +75,7 @@ double block_sum(const double* thread_vals) {
   return v;
 }
 
-// mdot_k<double> + reduce_partials_k: sum_i a[i] b[i]
+// mdot64_k: sum_i a[i] b[i]
 double gdot(int64_t n, const double* a, const double* b, int G) {
   std::vector<double> partial(G);
   const int64_t stride = int64_t(G) * kBlock;
@@ -267,7 +267,7 @@ struct Solver {
     }
   }
 
-  // maxpy_k: w -= sum_k h[k] V[k]; optionally ||w||^2 in the kernel's order
+  // maxpy64_k: w -= sum_k h[k] V[k]; optionally ||w||^2 in the kernel's order
   double maxpy(int nv, const double* V, const double* h, double* w, bool norm) const {
     const int64_t n = A.n;
 #pragma omp parallel for schedule(static)
