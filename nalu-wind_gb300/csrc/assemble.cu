@@ -37,6 +37,7 @@
 #include "schedule.h"
 #include "dd.h"
 #include "nw_internal.h"
+#include "row_stage.h"
 
 namespace nw {
 namespace {
@@ -737,7 +738,7 @@ __device__ __forceinline__ void row3_groups(int64_t g, int64_t step, int64_t fir
     if (r0 >= end_row) return b;
     const int64_t r1 = r0 + kRow3Group < end_row ? r0 + kRow3Group : end_row, r = r0 + trio;
     b.base = a.row_ptr[3 * r0];
-    b.cnt = int32_t(a.row_ptr[3 * r1] - b.base);
+    b.cnt = stage_count(b.base, a.row_ptr[3 * r1]);
     if (trio < kRow3Group && r < r1) {
       b.s = a.inc_ptr[r];
       b.t = a.inc_ptr[r + 1];
@@ -764,7 +765,7 @@ __device__ __forceinline__ void row3_groups(int64_t g, int64_t step, int64_t fir
     // the staged range keeps the parity of the CSR position, so that both
     // sides of the copy are 16-byte aligned together
     const int odd = int(b.base & 1);
-    const bool staged = (b.cnt + odd) * int(sizeof(double)) <= a.smem_bytes;
+    const bool staged = stage_fits(b.cnt, odd, a.smem_bytes);
     const bool acc = accumulate && !staged;
     double* v = staged ? stage + odd + (b.bq - b.base) : a.values + b.bq;
     if (s == t && trio < kRow3Group && r < end_row && !acc) {
