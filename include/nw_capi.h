@@ -296,10 +296,10 @@ nw_status nw_assemble_momentum_rows_range(nw_linsys* ls, const nw_momentum_opts*
  * the edge kernel writes every edge's coefficients to a buffer in HBM, then
  * the row kernel reads them back. SINGLE_KERNEL: one persistent kernel takes
  * edge chunks and node-row blocks from a fixed work list; the coefficients
- * pass through a ring of slots sized to stay in L2 (at most 64 MB), so they
- * never travel to DRAM (about 1.1x the compulsory bytes instead of 1.6x),
- * but on GB300 it runs slower than the two kernels (both phases are bound by
- * instruction issue, not by HBM). Both give the same CSR values and rhs, bit
+ * pass through a ring of slots sized for L2 (at most 64 MB), so most of them
+ * stay out of DRAM (1.4x the compulsory bytes instead of 1.65x at 128 x 128 x
+ * 64 hexes), but on GB300 it runs slower than the two kernels (both phases are
+ * bound by instruction issue, not by HBM). Both give the same CSR values and rhs, bit
  * for bit. A wait of the single kernel that times out (it cannot, by the
  * construction of the work list, but every wait is bounded) is reported as
  * NW_TIMEOUT by the next nw_linsys_sync, nw_linsys_copy_to_host or

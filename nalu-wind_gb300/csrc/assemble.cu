@@ -860,11 +860,19 @@ __global__ void __launch_bounds__(32 * kRow3Warps, kRow3PerSm) row3t_k(Row3Args 
 // ---------------------------------------------------------------------------
 // Single-kernel momentum assembly: a persistent kernel whose blocks take
 // edge chunks and row blocks from the work list of schedule.h in ticket
-// order. Edge chunks write their coefficients into a ring of slots small
-// enough to stay in L2, row blocks read them from there, so the coefficient
-// round trip of the two-kernel form never reaches DRAM. The arithmetic and
+// order. Edge chunks write their records into a ring of slots small enough
+// for L2 and row blocks read them from there, so that most of the record
+// round trip of the two-kernel form stays out of DRAM. The arithmetic and
 // the summation order are those of momentum_edge_k + row3t_k: the CSR
 // values are the same bits.
+//
+// Bound by its barriers and instruction issue. Three blocks a SM (80
+// registers, about 100 bytes of spills a thread): at four (64 registers) the
+// row part spills 370 bytes a thread, 57 MB over the resident threads, which
+// push the 50 MB ring out of L2. 128 x 128 x 64 hexes: 1.22 GB of DRAM traffic and
+// 613 us with three, 1.55 GB and 632 us with four (two kernels 1.45 GB and
+// 449 us); 734,831 edges of random tets, option set in full: 194 and 227 us.
+// Two blocks a SM take 791 and 186 us.
 //
 // Dependencies are flags holding the launch's generation number: a chunk's
 // flag is set once its coefficients are written, a row block's once its
@@ -924,8 +932,9 @@ __device__ bool wait_flags(const int* flags, const int32_t* list, int n, int gen
   return all;
 }
 
+constexpr int kFusedPerSm = 3;
 template <bool LIMITER, bool DIVU, bool DEF>
-__global__ void __launch_bounds__(kFusedChunk, 4)
+__global__ void __launch_bounds__(kFusedChunk, kFusedPerSm)
     momentum_fused_k(FusedArgs f, MomentumIn in, MomentumDD c, Row3Args ra, double* ring) {
   extern __shared__ double stage[];
   __shared__ int s_item[2];
