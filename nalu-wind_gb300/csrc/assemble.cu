@@ -1253,10 +1253,13 @@ int row_stage_bytes(int kind, const int64_t* row_ptr_host, int64_t R) {
     if (c > mx) mx = c;
   }
   // kind 2 and 3: bytes of one warp, one more entry so that the range can
-  // start at its parity, a multiple of 16
+  // start at its parity, a multiple of 16; at most its share of the block's.
+  // Rows beyond it are written entry by entry: 943,991 edges with 19 block
+  // columns a row took 267 us with 12 KB a warp of kind 2 (17 columns fit),
+  // 161 with its 16 KB (22 fit).
   if (kind >= 2) {
-    const int64_t most = kMaxRowSmem / (kFusedChunk / 32);
-    return int(std::min<int64_t>((mx + 2) / 2 * 16, most));
+    const int warps = kind == 2 ? kRow3Warps : kFusedChunk / 32;
+    return int(std::min<int64_t>((mx + 2) / 2 * 16, kMaxRowSmem / warps));
   }
   const int64_t bytes = mx * int64_t(sizeof(double));
   return bytes <= kMaxRowSmem ? int(bytes) : kMaxRowSmem;

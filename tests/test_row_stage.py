@@ -6,6 +6,7 @@ import ctypes
 import subprocess
 from pathlib import Path
 
+import numpy as np
 import pytest
 
 HERE = Path(__file__).resolve().parent
@@ -28,3 +29,19 @@ def test_staged_exactly_when_it_fits(lib):
         for first in (0, 1, 2 ** 33 + 1):
             for n in sizes:
                 assert bool(lib.row_staged(first, first + n, smem)) == (8 * (n + first % 2) <= smem), (smem, first, n)
+
+
+@pytest.mark.parametrize("columns", [7, 15, 17, 18, 20, 22])
+def test_momentum_rows_of_22_block_columns_are_staged(lib, nw, columns):
+    """The staging that the library gives a warp of the momentum row kernel
+    (six warps share a block's 96 KB: 16 KB each, 2,048 entries) holds ten
+    node rows of up to 22 block columns, whatever their position's parity."""
+    f = nw.load()._ZN2nw15row_stage_bytesEiPKll
+    f.restype, f.argtypes = ctypes.c_int, [ctypes.c_int, ctypes.c_void_p, ctypes.c_int64]
+    nodes = 37
+    row_ptr = np.arange(3 * nodes + 1, dtype=np.int64) * (3 * columns)
+    smem = f(2, row_ptr.ctypes.data, nodes)
+    assert smem % 16 == 0 and 6 * smem <= 96 * 1024
+    lib.row_staged.argtypes = [ctypes.c_int64, ctypes.c_int64, ctypes.c_int]
+    for first in (0, 1):
+        assert lib.row_staged(first, first + 10 * 9 * columns, smem)
