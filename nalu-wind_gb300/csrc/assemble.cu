@@ -581,7 +581,7 @@ __global__ void __launch_bounds__(kRow1Threads)
            double irelax, double* __restrict__ values, double* __restrict__ rhs,
            int accumulate, int smem_bytes) {
   using C = typename std::conditional<KIND == 0, double, dd>::type;
-  extern __shared__ double stage[];
+  extern __shared__ __align__(16) double stage[];
   const int64_t r0 = int64_t(blockIdx.x) * kRow1Threads;
   const int64_t r1 = (r0 + kRow1Threads < R) ? r0 + kRow1Threads : R;
   const int64_t base = row_ptr[r0];
@@ -851,7 +851,7 @@ __device__ __forceinline__ void row3_groups(int64_t g, int64_t step, int64_t fir
 
 template <typename IDX, int ACC>
 __global__ void __launch_bounds__(32 * kRow3Warps, kRow3PerSm) row3t_k(Row3Args a) {
-  extern __shared__ double stage[];
+  extern __shared__ __align__(16) double stage[];
   row3_groups<true, IDX, ACC>(int64_t(blockIdx.x) * kRow3Warps + (threadIdx.x >> 5),
                               int64_t(gridDim.x) * kRow3Warps, a.r_begin, a.R, a,
                               stage + (threadIdx.x >> 5) * (a.smem_bytes >> 3));
@@ -936,7 +936,7 @@ constexpr int kFusedPerSm = 3;
 template <bool LIMITER, bool DIVU, bool DEF>
 __global__ void __launch_bounds__(kFusedChunk, kFusedPerSm)
     momentum_fused_k(FusedArgs f, MomentumIn in, MomentumDD c, Row3Args ra, double* ring) {
-  extern __shared__ double stage[];
+  extern __shared__ __align__(16) double stage[];
   __shared__ int s_item[2];
   int next = 0;
   if (threadIdx.x == 0) next = atomicAdd(f.ticket, 1);
