@@ -33,6 +33,7 @@
 #include <cmath>
 #include <cstring>
 
+#include "gs_order.h"
 #include "krylov.h"
 #include "last_block.h"
 #include "learned.h"
@@ -781,7 +782,6 @@ __global__ void __launch_bounds__(kBlock)
 // fresh (forward from zero): the node's later rows still hold zero and are not
 // read. first (the first colour from zero): so do all other nodes; only the
 // node's earlier rows enter, at own[k], the first entry of the node's block.
-constexpr int kMaxDof = 3;
 constexpr int kGsNodeBatch = 20, kGsNodeBlock = 64;
 struct GsNodeArgs {
   int64_t cnt;
@@ -1547,32 +1547,29 @@ void KrylovSolver::sgs(const VT* vals, const T* rd, const T* x, T* y, cudaStream
   if (nc < 1) fail(NW_INTERNAL, "Gauss-Seidel colour classes not set up");
   // sweep 0: symmetric (forward then backward); 1: forward only; 2: backward only
   if (gs_dof_ > 1) {
-    const int dof = gs_dof_, ncol = nc / dof;
-    if (ncol > 2 && !from_guess) fill_k<T><<<grid1(A_.n), kBlock, 0, s>>>(A_.n, y, T(0));
-    auto node_pass = [&](int c, bool forward, bool backward, bool skip_last) {
+    const int dof = gs_dof_;
+    // the backward sweep from zero reads rows that gs_node_k does not know to be zero
+    if (!from_guess && (nc > 2 * dof || sweep == 2)) fill_k<T><<<grid1(A_.n), kBlock, 0, s>>>(A_.n, y, T(0));
+    gs_node_passes(nc / dof, dof, sweep, [&](const GsNodePass& p) {
       GsNodeArgs g{};
-      g.dof = dof;
-      g.cnt = gs_cptr_[c * dof + 1] - gs_cptr_[c * dof];
-      if (g.cnt == 0) return;
+      const int c = p.colour;
       const int64_t b = gs_cptr_[c * dof];
+      g.cnt = gs_cptr_[c * dof + 1] - b;
+      if (g.cnt == 0) return;
       g.rows = gs_rows_.p + b;
       g.len = gs_len_.p + b;
       g.own = gs_own_.p;
       g.off = gs_off_.p + gs_slice0_[c * dof];
       g.size = gs_size_[c];
-      if (forward)
-        for (int d = 0; d < dof; ++d) g.seq[g.nseq++] = d;
-      g.nfwd = g.nseq;
-      if (backward)
-        for (int d = dof - (skip_last ? 2 : 1); d >= 0; --d) g.seq[g.nseq++] = d;
+      g.dof = dof;
+      g.nseq = p.nseq;
+      g.nfwd = p.nfwd;
+      std::copy(p.seq, p.seq + p.nseq, g.seq);
       g.fresh = !from_guess;
       g.first = c == 0 && !from_guess;
       gs_node_k<VT, T><<<unsigned((g.cnt + kGsNodeBlock - 1) / kGsNodeBlock), kGsNodeBlock, 0, s>>>(
           g, gs_cols_.p, vals, rd, x, y);
-    };
-    // the row relaxed last by the forward sweep is not repeated
-    for (int c = 0; c < ncol; ++c) node_pass(c, true, c == ncol - 1, true);
-    for (int c = ncol - 2; c >= 0; --c) node_pass(c, false, true, false);
+    });
     NW_CUDA(cudaGetLastError());
     return;
   }
