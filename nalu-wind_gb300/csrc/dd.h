@@ -10,7 +10,8 @@
 //   add:  |err| <= 2 u^2 (|a| + |b|)      (relative to the operand sizes,
 //                                          not to the possibly cancelling sum)
 //   mul:  |err| <= 4 u^2 |a b|
-//   rcp:  |err| <= 3 u^2 / |x|            (one step from a float seed)
+//   rcp:  |err| <= 6 u^2 / |x|            (linear step from the float reciprocal)
+//   rcp_fast: |err| <= 4 u^2 / |x|        (quadratic step, any close seed)
 // Conversions from double keep the top 48 significand bits (the split error
 // is <= 2^-48 relative); dd -> double rounds hi + lo once. The
 // exponent range is the float range: |x| >= 2^128 becomes infinite, and
@@ -367,23 +368,31 @@ NW_HD dd dd_rcp(dd x) {
   const float e = fsub(fsub(1.0f, p), pe);
   return fast_two_sum(r0, fmul(r0, e));
 }
-// The same from the approximate float reciprocal (within 2^-22, a third of
-// the division's instructions) with a quadratic step r0 (1 + e + e^2), which
-// leaves the same error bound.
-NW_HD dd dd_rcp_fast(dd x) {
-  x = fast_two_sum(x.hi, x.lo);
-#ifdef __CUDA_ARCH__
-  float r0;
-  asm("rcp.approx.f32 %0, %1;" : "=f"(r0) : "f"(x.hi));
-#else
-  const float r0 = 1.0f / x.hi;
-#endif
-  if (x.hi == 0.0f || !(fabsf(r0) < INFINITY)) return {r0, 0.0f};
+// The same for |x.lo| <= ulp(x.hi) / 2 from any seed r within 2^-21 of 1 / x.hi:
+// a Newton step in single precision brings it to the nearest float, but for
+// ties, and the word step is quadratic, r0 (1 + e + e^2). Without the Newton
+// step the roundings of e, e + e^2 and their product grow with the seed's
+// distance (6.9 u^2 at one unit in the last place, 13 at 2^-22).
+NW_HD dd dd_rcp_seed(dd x, float r) {
+  if (x.hi == 0.0f || !(fabsf(r) < INFINITY)) return {r, 0.0f};
+  const float r0 = ffma(r, ffma(-x.hi, r, 1.0f), r);
   const float p = fmul(x.hi, r0);
   float pe = ffma(x.hi, r0, -p);
   pe = ffma(x.lo, r0, pe);
   const float e = fsub(fsub(1.0f, p), pe);
   return fast_two_sum(r0, fmul(r0, ffma(e, e, e)));
+}
+// from the approximate float reciprocal (one unit in the last place), a third
+// of the division's instructions
+NW_HD dd dd_rcp_fast(dd x) {
+  x = fast_two_sum(x.hi, x.lo);
+#ifdef __CUDA_ARCH__
+  float r;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(x.hi));
+#else
+  const float r = 1.0f / x.hi;
+#endif
+  return dd_rcp_seed(x, r);
 }
 
 NW_HD dd dd_abs(dd a) { return a.hi < 0.0f ? -a : a; }
