@@ -365,10 +365,11 @@ nw_status nw_linsys_copy_from_host(nw_linsys* ls, const double* values,
  * TpetraLinearSolver::solve (src/LinearSolver.C:209-254). x (device, nrows)
  * receives the solution from x0 = 0; final_iter selects final_tolerance.
  * Returns when the solve is done (the report needs its results). The GMRES
- * methods launch their iterations as CUDA graphs captured on the
- * handle's stream; on the legacy default stream, which cannot be captured,
- * the solve runs on a stream of the handle's own, ordered after earlier
- * work on the caller's stream and before later work by events. */
+ * methods launch their iterations as CUDA graphs, recorded on a stream of the
+ * handle's own: the handle's stream is never captured, and other threads may
+ * use it during a solve. On the legacy default stream the solve runs on a
+ * stream of the handle's own, ordered after earlier work on the caller's
+ * stream and before later work by events. */
 nw_status nw_linsys_solve(nw_linsys* ls, double* x, int final_iter,
                           nw_solve_report* rep);
 /* Residual history of the last solve (relative, first entry 1). */

@@ -1207,30 +1207,29 @@ KrylovSolver::Cycle KrylovSolver::run_cycle(int m, int max_steps, double g0, dou
   for (int j = 0; j < m && launched < max_steps && !stop;) {
     const int cnt = std::min({kChunk, m - j, max_steps - launched});
     const bool full = cnt == kChunk;
-    auto chunk = [&] {
+    auto chunk = [&](cudaStream_t to) {
       for (int k = 0; k < cnt; ++k)
         arnoldi(j + k, GivensCol{G, j + k, hs, hn, tol, div, hist_mul, hist_div,
-                                 full && k == cnt - 1 ? ctl_pinned_ + 4 * slot : nullptr});
+                                 full && k == cnt - 1 ? ctl_pinned_ + 4 * slot : nullptr}, to);
     };
     // A solve's first chunk runs as plain launches: any one-time set-up
     // (buffer growth) happens there, outside a capture. So does a shorter
-    // last chunk, which would not fit the graph, and every chunk on a stream
-    // that cannot be captured (the legacy default stream).
-    bool captured = graph && full && (set_up || j > 0);
-    if (captured && cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
-      cudaGetLastError();
-      graph = captured = false;
-    }
+    // last chunk, which would not fit the graph. The capture records on a
+    // stream of the solver's own, never on s: other threads may use the
+    // caller's stream during a solve, and their work would be captured too,
+    // their queries end the capture. The graph is launched on s.
+    const bool captured = graph && full && (set_up || j > 0);
     if (captured) {
       cudaGraph_t g = nullptr;
+      NW_CUDA(cudaStreamBeginCapture(capture_, cudaStreamCaptureModeThreadLocal));
       try {
-        chunk();
+        chunk(capture_);
       } catch (...) {
-        cudaStreamEndCapture(s, &g);
+        cudaStreamEndCapture(capture_, &g);
         if (g) cudaGraphDestroy(g);
         throw;
       }
-      NW_CUDA(cudaStreamEndCapture(s, &g));
+      NW_CUDA(cudaStreamEndCapture(capture_, &g));
       if (iter_exec_) {
         cudaGraphExecUpdateResultInfo info;
         if (cudaGraphExecUpdate(iter_exec_, g, &info) != cudaSuccess) {
@@ -1250,7 +1249,7 @@ KrylovSolver::Cycle KrylovSolver::run_cycle(int m, int max_steps, double g0, dou
       cudaGraphDestroy(g);
       NW_CUDA(cudaGraphLaunch(iter_exec_, s));
     } else {
-      chunk();
+      chunk(s);
     }
     j += cnt;
     launched += cnt;
@@ -1291,6 +1290,7 @@ void cycle_solution(double* gst, int* gctl, int m, int kk, double yscale, double
 // ---------------------------------------------------------------------------
 KrylovSolver::~KrylovSolver() {
   if (iter_exec_) cudaGraphExecDestroy(iter_exec_);
+  if (capture_) cudaStreamDestroy(capture_);
   if (h_pinned_) cudaFreeHost(h_pinned_);
   if (ctl_pinned_) cudaFreeHost(ctl_pinned_);
   for (cudaEvent_t& e : chunk_ev_)
@@ -1323,6 +1323,7 @@ void KrylovSolver::setup(const DevCsr& A, int m, cudaStream_t s) {
   if (!ctl_pinned_) NW_CUDA(cudaMallocHost(&ctl_pinned_, sizeof(int) * 12));
   for (cudaEvent_t& e : chunk_ev_)
     if (!e) NW_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  if (!capture_) NW_CUDA(cudaStreamCreateWithFlags(&capture_, cudaStreamNonBlocking));
   gst_.resize(size_t(m_ + 1) * m_ + 4 * size_t(m_) + 1);
   gctl_.resize(4);
   ticket_.resize(size_t(m_) / kTile + 2);
@@ -1991,7 +1992,7 @@ SolveResult KrylovSolver::gmres(const nw_solver_cfg& cfg, double tol,
     NW_CUDA(cudaMemcpyAsync(h2, &beta, sizeof(double), cudaMemcpyHostToDevice, s));
     scale_jacobi_k<double, false><<<grid1(n), kBlock, 0, s>>>(
         n, r_.p, V, h2, fuse_jacobi ? rdiag_.p : nullptr, flexible ? Z_.p : z_.p, GivensCol{});
-    auto arnoldi = [&](int j, const GivensCol& gc) {
+    auto arnoldi = [&](int j, const GivensCol& gc, cudaStream_t s) {
       double* vj = V + size_t(j) * n;
       double* zj = flexible ? Z_.p + size_t(j) * n : z_.p;
       if (!fuse_jacobi) apply_precond(pc, vj, zj, s);
@@ -2543,7 +2544,7 @@ SolveResult KrylovSolver::mixed(const nw_solver_cfg& cfg, double tol,
     scale_to_f32_k<<<grid1(n), kBlock, 0, s>>>(n, r_.p, V, h2);
     if (fuse_jacobi) jacobi_k<float><<<grid1(n), kBlock, 0, s>>>(n, rdiag32_.p, V, z32_.p);
     // inner system solved for r / ||r|| (g0 = 1)
-    auto arnoldi = [&](int j, const GivensCol& gc) {
+    auto arnoldi = [&](int j, const GivensCol& gc, cudaStream_t s) {
       float* vj = V + size_t(j) * ld;
       float* zj = flexible ? Z32_.p + size_t(j) * ld : z32_.p;
       if (!fuse_jacobi) precond32(pc, vj, zj, s);

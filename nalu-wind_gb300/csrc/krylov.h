@@ -162,8 +162,8 @@ class KrylovSolver {
     nw_status status = NW_OK;
     std::vector<double> hist;
   };
-  // One restart cycle's Arnoldi steps (arnoldi(j, column) launches iteration
-  // j's kernels: the new column in hs[0..j], its norm at hn[0], then the
+  // One restart cycle's Arnoldi steps (arnoldi(j, column, stream) launches
+  // iteration j's kernels: the new column in hs[0..j], its norm at hn[0], then the
   // column's Givens update beside the scaling of the new vector), with the
   // host one chunk behind.
   // With `graph`, chunks after the solve's first (set_up: an earlier cycle has
@@ -174,6 +174,7 @@ class KrylovSolver {
   Cycle run_cycle(int m, int max_steps, double g0, double tol, double div, double hist_mul, double hist_div,
                   StepFn arnoldi, const double* hs, const double* hn, cudaStream_t s, bool graph, bool set_up);
   cudaGraphExec_t iter_exec_ = nullptr;
+  cudaStream_t capture_ = nullptr;  // records the chunks; nothing runs on it
   // Sliced ELLPACK copy (slices of 32 rows, column-major within a slice)
   // used by the solver's SpMV: coalesced value/column loads for short rows.
   // sell_map_ holds the CSR index of every slot (-1 for padding).

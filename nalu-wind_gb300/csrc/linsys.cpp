@@ -89,8 +89,8 @@ struct nw_linsys {
   nw_solve_report last_report{};  // of the last solve (checkpointed)
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   // solves of a handle on the legacy default stream run on this stream
-  // (non-blocking, joined to the caller's stream by events), because the
-  // legacy stream cannot be captured into the solver's CUDA graphs
+  // (non-blocking, joined to the caller's stream by events): a legacy stream's
+  // launches wait for every blocking stream of the device
   cudaStream_t solve_stream = nullptr;
   cudaEvent_t solve_in = nullptr, solve_out = nullptr;
   bool timed = false;
