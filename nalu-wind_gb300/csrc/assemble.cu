@@ -30,6 +30,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdint>
 #include <type_traits>
 
@@ -102,8 +103,11 @@ __device__ __forceinline__ void ld32(const double* p, double (&x)[4]) {
 // takes one reciprocal for both of its divisions, the tanh form 0.5 (1 +
 // tanh x) is 1 / (1 + exp(-2 x)), and with alpha = 0 (the default) only the
 // upwind side is extrapolated and limited. 68 FP64 instructions an edge
-// against 132 (classic), 104 against 196 (limiter and tanh): 476,280 nodes
-// 576 -> 338 us with the row phase.
+// against 132 (classic), 105 against 196 (limiter and tanh): 476,280 nodes
+// 576 -> 333 us with the row phase. Errors of the entries against extended
+// precision (rms, 49 x 40 x 30 hexes, tanh and relax 0.7; 132 and 196
+// instructions and now): downwind side 1.88e-16 and 1.59e-16, upwind side
+// 8.5e-17 and 7.3e-17, diagonal 1.23e-16 and 1.20e-16.
 struct ScalarArgs {
   double alpha, alpha_upw, om_alpha, om_alpha_upw, upw, h, c1, k2;  // h = hf / 2, k2 = -2 / c2
 };
@@ -152,15 +156,18 @@ __global__ void __launch_bounds__(kScalarBlock)
   // mu / rho: from the node pre-pass, or (small systems) here from rho
   const double dsum = NODE ? dor[L] + dor[R]
                            : __dadd_rn(__dmul_rn(dflux[L], fast_rcp(dor[L])), __dmul_rn(dflux[R], fast_rcp(dor[R])));
-  const double den = fma(0.5, dsum, eps);
-  double pec;
+  double pec, om;  // Peclet function and one less it
   if (TANH) {
-    const double pe = (0.5 * fabs(udx)) * fast_rcp(den);
-    pec = fast_rcp(1.0 + exp((pe - o.c1) * o.k2));
+    const double pe = fabs(udx) * fast_rcp(dsum + 2.0 * eps);  // 0.5 |udx| over the mean diffusivity
+    const double ex = exp((pe - o.c1) * o.k2);
+    pec = fast_rcp(1.0 + ex);
+    // as a product: a difference would lose what the rounding of 1 + ex lost.
+    // ex may be infinite where pec is zero (tested on its bits)
+    om = __double_as_longlong(pec) == 0 ? 1.0 : ex * pec;
   } else {
-    const double u = o.h * udx, u2 = u * u;
+    const double den = fma(0.5, dsum, eps), u = o.h * udx, u2 = u * u;
     pec = u2 * fast_rcp(fma(5.0 * den, den, u2));
-
+    om = 1.0 - pec;
   }
   const double dq = qR - qL, qIp = 0.5 * (qL + qR);
   // lhsfac dq + non-orthogonal correction -visc / 2 (A - w dx) . (gL + gR)
@@ -168,7 +175,7 @@ __global__ void __launch_bounds__(kScalarBlock)
   const double diff = fma(lhsfac, dq, -(0.5 * visc) * fma(-w, dL + dR, ag));
   // upwind value - mean of the upwind side
   const double half = 0.5 * o.upw;
-  double qc = qIp, dU, m0, mc;
+  double qc = qIp, dU;
   if (!ALPHA) {
     const double dS = up ? dL : dR;
     double f = half * dS;
@@ -187,26 +194,34 @@ __global__ void __launch_bounds__(kScalarBlock)
   // adv = mdot (pec (a_u q_upw + (1 - a_u) qIp) + (1 - pec) q_cds)
   const double pa = pec * o.alpha_upw;  // weight of the upwind deviation
   const double mp = mdot * pa, hm = 0.5 * mdot;
-  double adv;
+  double adv, a01, a10;
   if (!ALPHA) {
     adv = fma(mp, dU, mdot * qIp);
-    m0 = 0.0;
-    mc = fma(-hm, pa, hm);  // mdot / 2 (1 - pec a_u)
+    if (TANH) {
+      // downwind side mdot / 2 (1 - pec a_u), upwind side mdot / 2 (1 + pec a_u)
+      const double sh = up ? hm : -hm;
+      const double dw = fma(sh, fma(o.alpha_upw, om, o.om_alpha_upw), lhsfac);
+      const double uw = lhsfac - fma(sh, pa, sh);
+      a01 = up ? dw : uw;
+      a10 = up ? uw : dw;
+    } else {
+      const double mc = fma(-hm, pa, hm);  // mdot / 2 (1 - pec a_u)
+      a01 = lhsfac + mc;
+      a10 = lhsfac - mc;
+    }
   } else {
-    const double om = 1.0 - pec;
     adv = fma(mp, dU, mdot * fma(pec, qIp, om * qc));
-    m0 = hm * o.alpha * om;
-    mc = hm * fma(pec, o.om_alpha_upw, om * o.om_alpha);
+    const double m0 = hm * o.alpha * om;
+    const double mc = hm * fma(pec, o.om_alpha_upw, om * o.om_alpha);
+    a01 = (lhsfac + mc) + m0;
+    a10 = (lhsfac - mc) - m0;
   }
-  double a01 = lhsfac + mc, a10 = lhsfac - mc;
-  if (ALPHA) {
-    a01 += m0;
-    a10 -= m0;
+  if (!TANH || ALPHA) {
+    if (up)
+      a10 -= mp;
+    else
+      a01 += mp;
   }
-  if (up)
-    a10 -= mp;
-  else
-    a01 += mp;
   st32(buf + kScalarCoefs * e, a01, a10, diff + adv, 0.0);
 }
 
@@ -578,7 +593,7 @@ __global__ void __launch_bounds__(kRow1Threads)
     row1_k(int64_t R, const int32_t* __restrict__ inc_ptr,
            const uint32_t* __restrict__ inc, const int32_t* __restrict__ diag_pos,
            const int64_t* __restrict__ row_ptr, const double* __restrict__ buf,
-           double irelax, double* __restrict__ values, double* __restrict__ rhs,
+           double irelax, double irelax_lo, double* __restrict__ values, double* __restrict__ rhs,
            int accumulate, int smem_bytes) {
   using C = typename std::conditional<KIND == 0, double, dd>::type;
   extern __shared__ __align__(16) double stage[];
@@ -636,7 +651,12 @@ __global__ void __launch_bounds__(kRow1Threads)
           acc_add(rra, cr);
         }
       }
-      if constexpr (KIND == 0) dg = -(dg * irelax);
+      if constexpr (KIND == 0) {
+        // dg / relax rounded once: 1 / relax as a pair (a rounded reciprocal left
+        // 1.28e-16 on the diagonal). An infinite sum takes no correction.
+        const bool finite = (__double2hiint(dg) & 0x7ff00000) != 0x7ff00000;
+        dg = -fma(dg, irelax, finite ? dg * irelax_lo : 0.0);
+      }
       if constexpr (KIND == 1) {
         dg = acc_value(dga);
         rr = acc_value(rra);
@@ -1272,12 +1292,14 @@ void launch_rows(cudaStream_t s, int kind, int64_t R, const int32_t* inc_ptr,
                  int smem_bytes, int max_inc, int64_t row_begin) {
   if (R <= row_begin) return;
   set_smem_attrs();
+  const double irelax = 1.0 / relax, lo = std::fma(-relax, irelax, 1.0) / relax;
   if (kind == 0)
     row1_k<0><<<grid_for(R, kRow1Threads), kRow1Threads, smem_bytes, s>>>(
-        R, inc_ptr, inc, diag_pos, row_ptr, buf, 1.0 / relax, values, rhs, accumulate, smem_bytes);
+        R, inc_ptr, inc, diag_pos, row_ptr, buf, irelax, std::isfinite(lo) ? lo : 0.0, values, rhs, accumulate,
+        smem_bytes);
   else if (kind == 1)
     row1_k<1><<<grid_for(R, kRow1Threads), kRow1Threads, smem_bytes, s>>>(
-        R, inc_ptr, inc, diag_pos, row_ptr, buf, 1.0, values, rhs, accumulate, smem_bytes);
+        R, inc_ptr, inc, diag_pos, row_ptr, buf, 1.0, 0.0, values, rhs, accumulate, smem_bytes);
   else {
     Row3Args a = row3_args(R, inc_ptr, inc, diag_pos, row_ptr, buf, relax, values, rhs, accumulate, smem_bytes);
     a.r_begin = row_begin;
