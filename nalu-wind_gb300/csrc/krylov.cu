@@ -1885,7 +1885,9 @@ void KrylovSolver::apply_precond(const Precond& pc, const double* x, double* y,
       pc.apply_fn(x, y, s);
       return;
     }
-    // FP64 interface around the FP32 learned preconditioner
+    // FP64 interface around the FP32 learned preconditioner, whatever the
+    // sweeps of the last solve read
+    gs_bf16_ = false;
     ensure_f32(s);
     const int64_t n = A_.n;
     tmp32b_.resize(n);
@@ -1921,6 +1923,7 @@ SolveResult KrylovSolver::solve(const nw_solver_cfg& cfg, double tol,
                                 const Precond& pc, const double* b, double* x,
                                 cudaStream_t s) {
   SolveResult r;
+  gs_bf16_ = cfg.precision == NW_PREC_MIXED_BF16;
   if (cfg.precision == NW_PREC_MIXED || cfg.precision == NW_PREC_MIXED_BF16)
     r = mixed(cfg, tol, pc, b, x, s);
   else if (cfg.method == NW_CG && pc.kind != NW_PC_LEARNED)
@@ -2505,7 +2508,6 @@ SolveResult KrylovSolver::mixed(const nw_solver_cfg& cfg, double tol,
                                 cudaStream_t s) {
   const int64_t n = A_.n;
   ensure_f32(s);
-  gs_bf16_ = cfg.precision == NW_PREC_MIXED_BF16;
   if (gs_bf16_) ensure_bf16(s);
   const int m = std::min(m_, std::max(1, cfg.inner_kspace > 0 ? cfg.inner_kspace : cfg.kspace));
   const double itol = cfg.inner_tolerance > 0 ? cfg.inner_tolerance : 1e-4;
