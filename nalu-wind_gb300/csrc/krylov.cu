@@ -1656,18 +1656,25 @@ void KrylovSolver::setup_colors(const std::vector<int32_t>& rows,
     // equal lengths (block graph), so its slices repeat class (colour, 0)'s
     bool nodes = true;
     for (int c = 0; c < nc && nodes; ++c) {
-      const int64_t b0 = cptr[c - c % dof], cnt = cptr[c + 1] - cptr[c];
-      nodes = cnt == cptr[c - c % dof + 1] - b0;
-      for (int64_t k = 0; k < cnt && nodes; ++k)
-        nodes = rows[b0 + k] % dof == 0 && rows[cptr[c] + k] == rows[b0 + k] + c % dof && len[cptr[c] + k] == len[b0 + k];
+      const int d = c % dof;
+      const int64_t b0 = cptr[c - d], b = cptr[c], cnt = cptr[c + 1] - b;
+      if (cnt != cptr[c - d + 1] - b0) {
+        nodes = false;
+        break;
+      }
+      bool other = false;  // no early exit: a pass over all rows, once a set-up
+      if (d == 0)
+        for (int64_t k = 0; k < cnt; ++k) other |= rows[b + k] % dof != 0;
+      else
+        for (int64_t k = 0; k < cnt; ++k) other |= (rows[b + k] != rows[b0 + k] + d) | (len[b + k] != len[b0 + k]);
+      nodes = !other;
     }
     if (nodes) {
       std::vector<int32_t> own(cptr[1]);  // only the first colour's is used
       for (int64_t k = 0; k < cptr[1]; ++k) {
         const int32_t i = rows[k];
-        int32_t q = 0;
-        for (int64_t p = A_.row_ptr_host[i]; p < A_.row_ptr_host[i + 1] && A_.col_idx_host[p] < i; ++p) ++q;
-        own[k] = q;
+        const int32_t* row = A_.col_idx_host + A_.row_ptr_host[i];
+        own[k] = int32_t(std::lower_bound(row, A_.col_idx_host + A_.row_ptr_host[i + 1], i) - row);
       }
       gs_own_.upload(own, s);
       gs_size_.resize(nc / dof);
