@@ -64,29 +64,31 @@ void build_fused_schedule(int64_t num_edges, int64_t rows, const int32_t* inc_pt
       s.block_hi[c] = std::max(s.block_hi[c], k);
     }
   }
-  // distinct (block, chunk) pairs, sorted both ways
+  // the distinct chunks of each row block, ascending, and the blocks of each
+  // chunk. A block's rows repeat few chunks, often in a row: sorting them by
+  // block costs a fraction of sorting all pairs at once
+  s.in_ptr.assign(size_t(s.blocks) + 1, 0);
+  s.out_ptr.assign(size_t(s.chunks) + 1, 0);
+  std::vector<int32_t> own;
+  for (int64_t k = 0; k < s.blocks; ++k) {
+    own.clear();
+    for (int64_t r = k * kFusedBlock; r < std::min(rows, (k + 1) * kFusedBlock); ++r)
+      for (int32_t q = inc_ptr[r]; q < inc_ptr[r + 1]; ++q) {
+        const int32_t c = int32_t(((inc[q] & 0x7fffffffu) >> 1) / kFusedChunk);
+        if (own.empty() || own.back() != c) own.push_back(c);
+      }
+    std::sort(own.begin(), own.end());
+    own.erase(std::unique(own.begin(), own.end()), own.end());
+    s.in.insert(s.in.end(), own.begin(), own.end());
+    s.in_ptr[k + 1] = int32_t(s.in.size());
+    for (int32_t c : own) ++s.out_ptr[c + 1];
+  }
+  for (int64_t c = 0; c < s.chunks; ++c) s.out_ptr[c + 1] += s.out_ptr[c];
+  s.out.resize(s.in.size());
   {
-    std::vector<int64_t> pairs;
-    for (int64_t r = 0; r < rows; ++r)
-      for (int32_t q = inc_ptr[r]; q < inc_ptr[r + 1]; ++q)
-        pairs.push_back((r / kFusedBlock) << 32 | (((inc[q] & 0x7fffffffu) >> 1) / kFusedChunk));
-    std::sort(pairs.begin(), pairs.end());
-    pairs.erase(std::unique(pairs.begin(), pairs.end()), pairs.end());
-    s.in_ptr.assign(size_t(s.blocks) + 1, 0);
-    s.out_ptr.assign(size_t(s.chunks) + 1, 0);
-    for (int64_t p : pairs) {
-      ++s.in_ptr[(p >> 32) + 1];
-      ++s.out_ptr[(p & 0xffffffff) + 1];
-    }
-    for (int64_t k = 0; k < s.blocks; ++k) s.in_ptr[k + 1] += s.in_ptr[k];
-    for (int64_t c = 0; c < s.chunks; ++c) s.out_ptr[c + 1] += s.out_ptr[c];
-    s.in.resize(pairs.size());
-    s.out.resize(pairs.size());
     std::vector<int32_t> pos(s.out_ptr.begin(), s.out_ptr.end() - 1);
-    for (size_t i = 0; i < pairs.size(); ++i) {
-      s.in[i] = int32_t(pairs[i] & 0xffffffff);  // block-major order
-      s.out[pos[pairs[i] & 0xffffffff]++] = int32_t(pairs[i] >> 32);
-    }
+    for (int64_t k = 0; k < s.blocks; ++k)
+      for (int32_t i = s.in_ptr[k]; i < s.in_ptr[k + 1]; ++i) s.out[pos[s.in[i]]++] = int32_t(k);
   }
   // running maxima: the last chunk read by blocks 0..k, the last block
   // reading chunks 0..c
