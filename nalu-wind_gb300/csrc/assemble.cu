@@ -993,7 +993,7 @@ __global__ void __launch_bounds__(kFusedChunk, kFusedPerSm)
 
 // applyDirichletBCs / resetRows: identity (or diag_value) rows. kResetLanes
 // lanes a row: one thread for a node's rows made one uncoalesced pass over its
-// 3 x 81 entries (14 us for the walls of a box of 24x20x12 hexes, 2.6 now).
+// entries, three rows of up to 18 on a hex wall (14 us for the walls of a box of 24x20x12 hexes, 2.6 now).
 constexpr int kResetLanes = 16;
 __global__ void __launch_bounds__(kThreads)
     reset_rows_k(int64_t n, const int64_t* __restrict__ nodes,
@@ -1170,9 +1170,13 @@ void launch_continuity_edges(cudaStream_t s, int64_t E, int64_t N,
                              double* nodebuf) {
   if (E == 0) return;
   // Small systems form the node records in the edge kernel (the same
-  // operations): a launch costs more than the repeated ones. With and without
-  // the pre-pass: 19 k edges 21.2 and 17.9 us, 267 k 32.5 and 30.0. Ranges keep
-  // the pre-pass, whose records later ranges read.
+  // operations): a launch costs more than the repeated ones. With the pre-pass
+  // and without it, hexes in row order: 21 k edges 21.1 and 17.7 us, 86 k 21.2
+  // and 19.0, 276 k 27.3 and 25.7, 507 k 35.2 and 35.4, 811 k 49.9 and 56.0,
+  // 3.2 M 145.7 and 187.9. Randomly numbered tets: 18 k 25.6 and 24.0, 82 k 27.3
+  // and 26.1, 274 k 35.9 and 37.2, 497 k 46.6 and 50.5, 3.2 M 235.0 and 299.5. The
+  // forms break even near 0.5 M edges on the first and 0.2 M on the second; the line
+  // lies between. Ranges keep the pre-pass, whose records later ranges read.
   launch_continuity_edge_range(s, 0, N, 0, E, edges, f, o, buf, nodebuf, E > 262144);
 }
 

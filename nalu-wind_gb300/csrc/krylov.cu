@@ -204,9 +204,10 @@ __device__ __forceinline__ double warp_sum(float s, float c) {
   return double(s) + double(c);
 }
 
-// The order is that of 256 strided per-thread sums followed by a binary tree
-// over the threads, whatever the number of warps that share the work.
-// one warp; thread slots t = lane + 32 i of the 256, result in lane 0. A
+// Fixed-order sums of G partials p[0..G): the order is that of 256 strided
+// per-thread sums followed by a binary tree over the threads, whatever the
+// number of warps that share the work.
+// One warp; thread slots t = lane + 32 i of the 256, result in lane 0. A
 // slot at or beyond G holds zero, so levels that would only add zeros are
 // skipped.
 __device__ __noinline__ double warp_tree_sum(int G, const double* p) {
@@ -1038,6 +1039,7 @@ __device__ __forceinline__ float rn_div(float a, float b) { return __fdiv_rn(a, 
 // nodes: 19.5 ms with blocks of 256 and an entry at a time, 13.6, 13.1 and 11.7
 // with blocks of 128, 64 and 32.
 constexpr int kLevelBlock = 32;
+unsigned level_grid(int64_t rows) { return unsigned((rows + kLevelBlock - 1) / kLevelBlock); }
 template <typename VT, typename T>
 __global__ void __launch_bounds__(kLevelBlock)
     gs_level_k(int64_t cnt, const int32_t* __restrict__ rows, const int64_t* __restrict__ rp,
@@ -1579,8 +1581,7 @@ void KrylovSolver::sgs(const VT* vals, const T* rd, const T* x, T* y, cudaStream
     const int64_t b = gs_cptr_[c], cnt = gs_cptr_[c + 1] - b;
     if (cnt)
       pdl_launch(gs_sell_k<VT, T>, grid1(cnt), kBlock, 0, s, cnt, gs_rows_.p + b, gs_off_.p + gs_slice0_[c],
-                                                     gs_len_.p + b, gs_cols_.p, vals, rd, x, y,
-                                                     first);
+                 gs_len_.p + b, gs_cols_.p, vals, rd, x, y, first);
   };
   if (sweep == 2) {
     for (int c = nc - 1; c >= 0; --c) pass(c, c == nc - 1 && !from_guess);
@@ -1605,8 +1606,7 @@ void KrylovSolver::sgs_residual32(const float* x, const float* y, float* r, cuda
     const int64_t b = gs_cptr_[c], cnt = c == last ? 0 : gs_cptr_[c + 1] - b;
     if (cnt + zcnt)
       pdl_launch(gs_resid_k, grid1(cnt + zcnt), kBlock, 0, s, cnt, gs_rows_.p + b, gs_off_.p + gs_slice0_[c],
-                                                      gs_len_.p + b, gs_cols_.p, gs_vals32_.p, diag32_.p,
-                                                      x, y, r, zcnt, zrows);
+                 gs_len_.p + b, gs_cols_.p, gs_vals32_.p, diag32_.p, x, y, r, zcnt, zrows);
     zcnt = 0;
   }
   NW_CUDA(cudaGetLastError());
@@ -1792,8 +1792,8 @@ void KrylovSolver::sgs_natural(const VT* vals, const T* x, T* y, cudaStream_t s)
     for (size_t l = 0; l + 1 < ptr.size(); ++l) {
       const int64_t cnt = ptr[l + 1] - ptr[l];
       if (cnt)
-        pdl_launch(gs_level_k<VT, T>, unsigned((cnt + kLevelBlock - 1) / kLevelBlock), kLevelBlock, 0, s, cnt, rows + ptr[l], A_.row_ptr, A_.col_idx, vals,
-                                                         dpos_.p, x, y, pass == 0);
+        pdl_launch(gs_level_k<VT, T>, level_grid(cnt), kLevelBlock, 0, s, cnt, rows + ptr[l], A_.row_ptr,
+                   A_.col_idx, vals, dpos_.p, x, y, pass == 0);
     }
   }
   NW_CUDA(cudaGetLastError());
@@ -1821,14 +1821,14 @@ void KrylovSolver::ilu0_solve(const T* lu, const T* x, T* y, cudaStream_t s) {
   for (size_t l = 0; l + 1 < fl_ptr_.size(); ++l) {
     const int64_t cnt = fl_ptr_[l + 1] - fl_ptr_[l];
     if (cnt)
-      pdl_launch(ilu0_solve_level_k<false, T>, unsigned((cnt + kLevelBlock - 1) / kLevelBlock), kLevelBlock, 0, s, cnt, fl_rows_.p + fl_ptr_[l], A_.row_ptr,
-                                                                  A_.col_idx, dpos_.p, lu, x, y);
+      pdl_launch(ilu0_solve_level_k<false, T>, level_grid(cnt), kLevelBlock, 0, s, cnt, fl_rows_.p + fl_ptr_[l],
+                 A_.row_ptr, A_.col_idx, dpos_.p, lu, x, y);
   }
   for (size_t l = 0; l + 1 < bl_ptr_.size(); ++l) {
     const int64_t cnt = bl_ptr_[l + 1] - bl_ptr_[l];
     if (cnt)
-      pdl_launch(ilu0_solve_level_k<true, T>, unsigned((cnt + kLevelBlock - 1) / kLevelBlock), kLevelBlock, 0, s, cnt, bl_rows_.p + bl_ptr_[l], A_.row_ptr,
-                                                                 A_.col_idx, dpos_.p, lu, y, y);
+      pdl_launch(ilu0_solve_level_k<true, T>, level_grid(cnt), kLevelBlock, 0, s, cnt, bl_rows_.p + bl_ptr_[l],
+                 A_.row_ptr, A_.col_idx, dpos_.p, lu, y, y);
   }
   NW_CUDA(cudaGetLastError());
 }

@@ -1045,7 +1045,7 @@ void LearnedNet::forward(const CoarseLevel& cl, const float* wgt, const float* d
   const unsigned gw = gridn(nc * 32);  // warp per row
   pdl_launch(input_k, gridn(nc), kB, 0, s, nc, rc, dinv, work.u.p, work.partial.p, work.scal.p, work.ticket.p);
   pdl_launch(layer0_k, gw, kB, 0, s, nc, cl.cptr.p, cl.ccol.p, cl.cdiag.p, wgt, work.u.p, work.scal.p,
-                             params.p + kOffW0, work.x.p, work.ax.p, work.xc1.p);
+             params.p + kOffW0, work.x.p, work.ax.p, work.xc1.p);
   uint16_t* xcs[4] = {work.xc1.p, work.xc2.p, work.xc3.p, nullptr};
   for (int l = 0; l < 3; ++l) {
     pdl_launch(agg_fwd_k, gw, kB, 0, s, nc, cl.cptr.p, cl.ccol.p, cl.cdiag.p, wgt, xcs[l]);
@@ -1064,13 +1064,13 @@ void LearnedNet::coarse_correction(const CoarseLevel& cl, const float* rc, float
   } else {
     work.resize(cl.nc, s);
     pdl_launch(coarse_jacobi_k, nb, kB, 0, s, cl.nc, cl.cptr.p, cl.ccol.p, cl.cdiag.p, cl.wgt.p, cl.dinv.p, rc,
-                                      nullptr, coarse_mode == 1 ? ec : work.u.p);
+               nullptr, coarse_mode == 1 ? ec : work.u.p);
     if (coarse_mode == 2)
       pdl_launch(coarse_jacobi_k, nb, kB, 0, s, cl.nc, cl.cptr.p, cl.ccol.p, cl.cdiag.p, cl.wgt.p, cl.dinv.p, rc,
-                                        work.u.p, ec);
+                 work.u.p, ec);
   }
-  pdl_launch(coarse_apply_k, gridn(cl.nc, kRowBlock), kB, 0, s, cl.nc, cl.cptr.p, cl.ccol.p, cl.cdiag.p, cl.wgt.p, cl.dinv.p,
-                                   ec, rc, work.aec.p, work.partial.p, work.scal.p, work.ticket.p);
+  pdl_launch(coarse_apply_k, gridn(cl.nc, kRowBlock), kB, 0, s, cl.nc, cl.cptr.p, cl.ccol.p, cl.cdiag.p, cl.wgt.p,
+             cl.dinv.p, ec, rc, work.aec.p, work.partial.p, work.scal.p, work.ticket.p);
   NW_CUDA(cudaGetLastError());
 }
 
@@ -1084,7 +1084,7 @@ double LearnedNet::forward_backward(const CoarseLevel& cl, const float* wgt,
   const unsigned gw = gridn(nc * 32);
   const int nb = int(gridn(nc));
   pdl_launch(coarse_apply_k, gridn(nc, kRowBlock), kB, 0, s, nc, cl.cptr.p, cl.ccol.p, cl.cdiag.p, wgt, dinv, ec, rc,
-                                   work.aec.p, work.partial.p, work.scal.p, work.ticket.p);
+             work.aec.p, work.partial.p, work.scal.p, work.ticket.p);
   float sc[4];
   NW_CUDA(cudaMemcpyAsync(sc, work.scal.p, sizeof(sc), cudaMemcpyDeviceToHost, s));
   NW_CUDA(cudaStreamSynchronize(s));

@@ -15,10 +15,12 @@ namespace nw {
 // the one before).
 //
 // It pays for chains of short kernels bound by latency: the learned cycle (9.09
-// -> 8.53 ms for 90 iterations) and the level-scheduled sweeps (22.4 -> 18.6 ms
-// for 43x64x43 nodes, their levels then still in blocks of 256). The multi-dots, multi-axpys and scalings lost by it (32^3
-// GMRES 1.38 -> 1.57 ms, 1.08 M rows 17.4 -> 18.8 ms), the node sweeps too (1.55
-// -> 1.58 ms), and the matrix product gained nothing: they are launched plainly.
+// -> 8.53 ms for 90 iterations), its network layers' product included, and the
+// level-scheduled sweeps (22.4 -> 18.6 ms for 43x64x43 nodes, their levels then
+// still in blocks of 256). The multi-dots, multi-axpys and scalings lost by it
+// (32^3 GMRES 1.38 -> 1.57 ms, 1.08 M rows 17.4 -> 18.8 ms), the node sweeps too
+// (1.55 -> 1.58 ms), and the sparse product with the system's matrix gained
+// nothing: they are launched plainly.
 //
 // pdl_wait takes the pointers to such memory and hands them back through an
 // opaque statement behind the wait: a load through a const __restrict__
