@@ -1217,21 +1217,23 @@ KrylovSolver::Cycle KrylovSolver::run_cycle(int m, int max_steps, double g0, dou
     // A solve's first chunk runs as plain launches: any one-time set-up
     // (buffer growth) happens there, outside a capture. So does a shorter
     // last chunk, which would not fit the graph. The capture records on a
-    // stream of the solver's own, never on s: other threads may use the
-    // caller's stream during a solve, and their work would be captured too,
-    // their queries end the capture. The graph is launched on s.
+    // private stream, never on a caller's s: other threads may use that
+    // during a solve, and their work would be captured too, their queries
+    // end the capture. The graph is launched on s.
     const bool captured = graph && full && (set_up || j > 0);
     if (captured) {
       cudaGraph_t g = nullptr;
-      NW_CUDA(cudaStreamBeginCapture(capture_, cudaStreamCaptureModeThreadLocal));
+      if (!record_ && !own_record_) NW_CUDA(cudaStreamCreateWithFlags(&own_record_, cudaStreamNonBlocking));
+      const cudaStream_t rec = record_ ? record_ : own_record_;
+      NW_CUDA(cudaStreamBeginCapture(rec, cudaStreamCaptureModeThreadLocal));
       try {
-        chunk(capture_);
+        chunk(rec);
       } catch (...) {
-        cudaStreamEndCapture(capture_, &g);
+        cudaStreamEndCapture(rec, &g);
         if (g) cudaGraphDestroy(g);
         throw;
       }
-      NW_CUDA(cudaStreamEndCapture(capture_, &g));
+      NW_CUDA(cudaStreamEndCapture(rec, &g));
       if (iter_exec_) {
         cudaGraphExecUpdateResultInfo info;
         if (cudaGraphExecUpdate(iter_exec_, g, &info) != cudaSuccess) {
@@ -1292,7 +1294,7 @@ void cycle_solution(double* gst, int* gctl, int m, int kk, double yscale, double
 // ---------------------------------------------------------------------------
 KrylovSolver::~KrylovSolver() {
   if (iter_exec_) cudaGraphExecDestroy(iter_exec_);
-  if (capture_) cudaStreamDestroy(capture_);
+  if (own_record_) cudaStreamDestroy(own_record_);
   if (h_pinned_) cudaFreeHost(h_pinned_);
   if (ctl_pinned_) cudaFreeHost(ctl_pinned_);
   for (cudaEvent_t& e : chunk_ev_)
@@ -1325,7 +1327,6 @@ void KrylovSolver::setup(const DevCsr& A, int m, cudaStream_t s) {
   if (!ctl_pinned_) NW_CUDA(cudaMallocHost(&ctl_pinned_, sizeof(int) * 12));
   for (cudaEvent_t& e : chunk_ev_)
     if (!e) NW_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-  if (!capture_) NW_CUDA(cudaStreamCreateWithFlags(&capture_, cudaStreamNonBlocking));
   gst_.resize(size_t(m_ + 1) * m_ + 4 * size_t(m_) + 1);
   gctl_.resize(4);
   ticket_.resize(size_t(m_) / kTile + 2);

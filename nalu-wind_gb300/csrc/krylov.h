@@ -109,6 +109,9 @@ class KrylovSolver {
     cl_ = cl;
   }
   bool has_learned() const { return net_ && cl_; }
+  // A stream that nobody else uses, for recording graphs (else the solver
+  // makes its own when it first records one: 2 ms).
+  void record_on(cudaStream_t s) { record_ = s; }
   void ensure_f32(cudaStream_t s);
   void ensure_bf16(cudaStream_t s);  // after ensure_f32
   // FP32 preconditioner application (Jacobi, SGS or learned) of the mixed
@@ -174,7 +177,8 @@ class KrylovSolver {
   Cycle run_cycle(int m, int max_steps, double g0, double tol, double div, double hist_mul, double hist_div,
                   StepFn arnoldi, const double* hs, const double* hn, cudaStream_t s, bool graph, bool set_up);
   cudaGraphExec_t iter_exec_ = nullptr;
-  cudaStream_t capture_ = nullptr;  // records the chunks; nothing runs on it
+  cudaStream_t record_ = nullptr;      // private stream that records the chunks
+  cudaStream_t own_record_ = nullptr;  // the same when the owner gave none
   // Sliced ELLPACK copy (slices of 32 rows, column-major within a slice)
   // used by the solver's SpMV: coalesced value/column loads for short rows.
   // sell_map_ holds the CSR index of every slot (-1 for padding).

@@ -846,6 +846,7 @@ nw_status nw_linsys_solve(nw_linsys* ls, double* x, int final_iter,
       NW_CUDA(cudaEventRecord(ls->solve_in, ls->stream));
       NW_CUDA(cudaStreamWaitEvent(ls->solve_stream, ls->solve_in, 0));
       s = ls->solve_stream;
+      ls->solver.record_on(s);
     }
     SolveResult r;
     try {
