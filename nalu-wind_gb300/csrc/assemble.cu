@@ -687,7 +687,10 @@ __global__ void __launch_bounds__(kRow1Threads)
 // byte loads of the same words cost five times the L1 lookups), sums its own
 // entry of N and takes the other one it stores from the node's next lane.
 // The next record is loaded while one is summed. A warp stages its CSR range in
-// shared memory and writes it with one bulk copy. What it reads and writes (96
+// shared memory and writes it with one bulk copy, or adds it with one where the
+// system holds values: read, added and written by the lanes, repeated assembly of
+// 128 x 128 x 64 took 782 us (766 with the kernels of a block a range), 517 now, of
+// 1,167,183 tet edges 357 and 229. What it reads and writes (96
 // bytes an edge, the matrix) takes 125 us at 128 x 128 x 64; it takes 172,
 // with FP64 pipe, issue and L1 each about half busy (24 warps a SM without
 // spills measured the same as 36 with).
@@ -715,14 +718,20 @@ __device__ __forceinline__ void add64(double* p, double x) {
   *p = y;
 }
 
-// Bulk copy of `bytes` (a multiple of 16) from shared to global memory, both
-// 16-byte aligned, by one thread after the others' writes have been fenced
+// Bulk copy (add: element-wise addition to what is there, rounded as any other)
+// of `bytes` (a multiple of 16) from shared to global memory, both 16-byte
+// aligned, by one thread after the others' writes have been fenced
 // (fence_async) and joined.
 __device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void bulk_store(double* dst, const double* src, int bytes) {
-  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst),
-               "r"(uint32_t(__cvta_generic_to_shared(src))), "r"(bytes)
-               : "memory");
+__device__ __forceinline__ void bulk_store(double* dst, const double* src, int bytes, bool add) {
+  if (add)
+    asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f64 [%0], [%1], %2;" ::"l"(dst),
+                 "r"(uint32_t(__cvta_generic_to_shared(src))), "r"(bytes)
+                 : "memory");
+  else
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst),
+                 "r"(uint32_t(__cvta_generic_to_shared(src))), "r"(bytes)
+                 : "memory");
   asm volatile("cp.async.bulk.commit_group;" ::: "memory");
 }
 // the calling thread's bulk copies have read their sources
@@ -847,19 +856,13 @@ __device__ __forceinline__ void row3_groups(int64_t g, int64_t step, int64_t fir
     if (staged) {
       double* out = a.values + b.base - odd;
       const int end = b.cnt + odd;
-      if (!accumulate) {
-        // the whole 16-byte pairs as one bulk copy, the ends by hand
-        fence_async();
-        __syncwarp();
-        if (lane == 1 && odd && end > 1) out[1] = stage[1];
-        if (lane == 2 && (end & 1) && end > odd) out[end - 1] = stage[end - 1];
-        const int from = 2 * odd, bytes = ((end & ~1) - from) * int(sizeof(double));
-        if (lane == 0 && bytes > 0) bulk_store(out + from, stage + from, bytes);
-      } else {
-        __syncwarp();
-        for (int k = odd + lane; k < end; k += 32) out[k] += stage[k];
-        __syncwarp();
-      }
+      // the whole 16-byte pairs as one bulk copy, the ends by hand
+      fence_async();
+      __syncwarp();
+      const int by_hand = lane == 1 && odd && end > 1 ? 1 : (lane == 2 && (end & 1) && end > odd ? end - 1 : -1);
+      if (by_hand >= 0) out[by_hand] = accumulate ? out[by_hand] + stage[by_hand] : stage[by_hand];
+      const int from = 2 * odd, bytes = ((end & ~1) - from) * int(sizeof(double));
+      if (lane == 0 && bytes > 0) bulk_store(out + from, stage + from, bytes, accumulate);
     }
     if (first + g * kRow3Group >= end_row) {
       if (lane == 0) bulk_wait();
