@@ -12,11 +12,14 @@
 namespace nw {
 namespace {
 
-// Small blocks: a system of some thousand nodes then reaches every SM, and a
-// node's FP64 chains and divisions (64 clocks an instruction of a warp) have
-// the pipe to themselves: 8.3 us with blocks of 256 on 6,825 momentum nodes, 6.1
-// with 64.
-constexpr int kThreads = 64;
+// Systems of some thousand nodes take small blocks: they then reach every SM, and
+// a node's FP64 chains and divisions (64 clocks an instruction of a warp) have
+// the pipe to themselves. Momentum time term with blocks of 256 and 64: 990
+// nodes 10.4 and 8.2 us, 10,500 10.6 and 10.0, 14,175 11.3 and 11.1, 29,822 17.3
+// and 19.4, 172,032 64.7 and 65.2 (scalar 64.4 and 69.6), 1,081,665 360.9 and 365.5;
+// the diagonal of 172,032 4.2 and 6.2. The line lies between 14 and 30 thousand.
+constexpr int kThreads = 256, kSmallBlock = 64;
+constexpr int64_t kSmallNodes = 16384;
 
 // KIND 0: ScalarMassBDFNodeKernel::execute
 //         (src/node_kernels/ScalarMassBDFNodeKernel.C:75-97)
@@ -96,14 +99,15 @@ __global__ void udiag_post_k(int64_t n, const double* __restrict__ rho,
   udiag[i] = (u - pts) * alpha + pts;
 }
 
-inline unsigned grid_for(int64_t n) { return unsigned((n + kThreads - 1) / kThreads); }
+inline unsigned block_for(int64_t n) { return n <= kSmallNodes ? kSmallBlock : kThreads; }
+inline unsigned grid_for(int64_t n) { return unsigned((n + block_for(n) - 1) / block_for(n)); }
 
 }  // namespace
 
 void launch_extract_diagonal(cudaStream_t s, const PlanView& v, int dof, const double* values,
                              double* diag) {
   if (v.num_nodes == 0) return;
-  extract_diag_k<<<grid_for(v.num_nodes), kThreads, 0, s>>>(v.num_nodes, v.node_lid, v.num_dof, dof,
+  extract_diag_k<<<grid_for(v.num_nodes), block_for(v.num_nodes), 0, s>>>(v.num_nodes, v.node_lid, v.num_dof, dof,
                                                              v.diag_pos, v.row_ptr, values, diag);
   NW_CUDA(cudaGetLastError());
 }
@@ -111,7 +115,7 @@ void launch_extract_diagonal(cudaStream_t s, const PlanView& v, int dof, const d
 void launch_udiag_postprocess(cudaStream_t s, int64_t n, const double* rho, const double* dvol,
                               double pts, double alpha, double* udiag) {
   if (n == 0) return;
-  udiag_post_k<<<grid_for(n), kThreads, 0, s>>>(n, rho, dvol, pts, alpha, udiag);
+  udiag_post_k<<<grid_for(n), block_for(n), 0, s>>>(n, rho, dvol, pts, alpha, udiag);
   NW_CUDA(cudaGetLastError());
 }
 
@@ -119,13 +123,13 @@ void launch_mass_bdf(cudaStream_t s, int kind, const PlanView& v, const nw_mass_
                      const nw_bdf_opts& o, double* values, double* rhs) {
   if (v.node_rows == 0) return;
   if (kind == 0)
-    mass_bdf_k<0><<<grid_for(v.node_rows), kThreads, 0, s>>>(
+    mass_bdf_k<0><<<grid_for(v.node_rows), block_for(v.node_rows), 0, s>>>(
         v.node_rows, v.row_nodes_ptr, v.row_nodes, v.diag_pos, v.row_ptr, f, o, values, rhs);
   else if (kind == 1)
-    mass_bdf_k<1><<<grid_for(v.node_rows), kThreads, 0, s>>>(
+    mass_bdf_k<1><<<grid_for(v.node_rows), block_for(v.node_rows), 0, s>>>(
         v.node_rows, v.row_nodes_ptr, v.row_nodes, v.diag_pos, v.row_ptr, f, o, values, rhs);
   else
-    mass_bdf_k<2><<<grid_for(v.node_rows), kThreads, 0, s>>>(
+    mass_bdf_k<2><<<grid_for(v.node_rows), block_for(v.node_rows), 0, s>>>(
         v.node_rows, v.row_nodes_ptr, v.row_nodes, v.diag_pos, v.row_ptr, f, o, values, rhs);
   NW_CUDA(cudaGetLastError());
 }
