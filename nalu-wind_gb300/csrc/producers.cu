@@ -32,13 +32,17 @@ __device__ __forceinline__ dd ldd(const double* p) { return dd_from_double(*p); 
 //
 // Bound by instruction issue: products stay in float pairs, but sums of FP64
 // inputs and rho u are formed in FP64 (ten operations an edge on the
-// otherwise idle pipe), each split once. PLAIN: noc = interp = 1. It also waits
-// for the gathers of two random nodes: twelve blocks of 128 (40 registers) took
-// the four producers on 1,167,183 edges of tets from 144 us (four of 256) to
-// 137.6; ten 138.2, fourteen 141.6.
+// otherwise idle pipe), each split once. NOC1, TOG1: noc = 1, interp = 1, whose
+// terms with 1 - noc and 1 - interp are left out. It also waits for the gathers of
+// two random nodes: twelve blocks of 128 (40 registers) took the four producers
+// on 1,167,183 edges of tets from 144 us (four of 256) to 137.6; ten 138.2,
+// fourteen 141.6. The terms with 1 - noc need 54
+// registers, eight blocks: 3.2 M edges of hexes in row order take 109 us with the
+// default factors, 127 with noc 0.3, 117 with interp 0.4 (176 for these two as one
+// general form with twelve blocks; 152 for each before sums went to FP64).
 constexpr int kMdotBlock = 128;
-template <bool PLAIN>
-__global__ void __launch_bounds__(kMdotBlock, 12)
+template <bool NOC1, bool TOG1>
+__global__ void __launch_bounds__(kMdotBlock, NOC1 ? 12 : 8)
     mdot_k(int64_t E, const int2* __restrict__ edges, const double* __restrict__ coords,
            const double* __restrict__ velocity, const double* __restrict__ Gpdx,
            const double* __restrict__ density, const double* __restrict__ pressure,
@@ -48,7 +52,12 @@ __global__ void __launch_bounds__(kMdotBlock, 12)
   if (e >= E) return;
   const int2 lr = edges[e];
   const int64_t L = lr.x, R = lr.y;
-  const double rhoL = density[L], rhoR = density[R];
+  double rhoL = density[L], rhoR = density[R];
+  if (!TOG1) {  // 2 (interp rhoU_Ip + (1 - interp) rho_Ip u_Ip) is linear in u_L and u_R
+    const double h = om_interp * 0.5 * (rhoL + rhoR);
+    rhoL = fma(interp, rhoL, h);
+    rhoR = fma(interp, rhoR, h);
+  }
   const dd iuL = dd_rcp_fast(ldd(udiag + L)), iuR = dd_rcp_fast(ldd(udiag + R));
   dd av[3], dx[3], m[3], g[3];  // m = 2 rhoU_Ip, g = 2 G_Ip
 #pragma unroll
@@ -56,9 +65,7 @@ __global__ void __launch_bounds__(kMdotBlock, 12)
     av[d] = dd_from_double_near_z(area[3 * e + d]);
     dx[d] = dd_from_double_z(coords[3 * R + d] - coords[3 * L + d]);
     const double uL = velocity[3 * L + d], uR = velocity[3 * R + d];
-    double ru = fma(rhoR, uR, rhoL * uL);
-    if (!PLAIN) ru = fma(interp, ru, (om_interp * 0.5 * (rhoL + rhoR)) * (uL + uR));
-    m[d] = dd_from_double_near(ru);
+    m[d] = dd_from_double_near(fma(rhoR, uR, rhoL * uL));
     g[d] = ldd(Gpdx + 3 * R + d) * iuR + ldd(Gpdx + 3 * L + d) * iuL;
   }
   const dd asq = dd_dot3(av[0], av[0], av[1], av[1], av[2], av[2]);
@@ -66,10 +73,10 @@ __global__ void __launch_bounds__(kMdotBlock, 12)
   const dd w = asq * dd_rcp_fast(axdx);
   const dd ma = dd_dot3(m[0], av[0], m[1], av[1], m[2], av[2]);
   dd xg = dd_dot3(dx[0], g[0], dx[1], g[1], dx[2], g[2]);
-  if (!PLAIN) xg = noc * xg;
+  if (!NOC1) xg = noc * xg;
   // twice tmdot
   dd t = w * (xg - (iuL + iuR) * dd_from_double(pressure[R] - pressure[L])) + ma;
-  if (!PLAIN) t = om_noc * dd_dot3(g[0], av[0], g[1], av[1], g[2], av[2]) + t;
+  if (!NOC1) t = om_noc * dd_dot3(g[0], av[0], g[1], av[1], g[2], av[2]) + t;
   mdot[e] = dd_to_double_int(scale2(t, 0.5f));
 }
 
@@ -228,10 +235,10 @@ extern "C" nw_status nw_compute_mdot_edges(nw_linsys* ls, const nw_continuity_fi
           v.num_edges, v.edges, f->coords, f->velocity, f->dpdx, f->density, f->pressure, f->udiag, f->area,
           dd_from_double(noc_fac), dd_from_double(1.0 - noc_fac), interp_together, 1.0 - interp_together, mdot);
     };
-    if (noc_fac == 1.0 && interp_together == 1.0)
-      go(nw::mdot_k<true>);
+    if (noc_fac == 1.0)
+      interp_together == 1.0 ? go(nw::mdot_k<true, true>) : go(nw::mdot_k<true, false>);
     else
-      go(nw::mdot_k<false>);
+      interp_together == 1.0 ? go(nw::mdot_k<false, true>) : go(nw::mdot_k<false, false>);
     NW_CUDA(cudaGetLastError());
   });
 }
