@@ -184,14 +184,17 @@ __global__ void __launch_bounds__(kThreads)
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
     dx[d] = scale2(dd_from_double_near_z(coords[3 * R + d] - coords[3 * L + d]), 0.5f);
-    us[d] = dd_from_double_near(vel[3 * R + d] + vel[3 * L + d]);
+    // one FP64 addition and a split; with the tanh form, which fills the FP64
+    // pipe, two splits and a pair addition
+    us[d] = o.tanh_form ? ldd(vel + 3 * R + d) + ldd(vel + 3 * L + d)
+                        : dd_from_double_near(vel[3 * R + d] + vel[3 * L + d]);
   }
   const dd udotx = dd_dot3(dx[0], us[0], dx[1], us[1], dx[2], us[2]);
   const dd pe = dd_abs(udotx) * dd_rcp_fast(diffIp + eps);
   if (pecnum) pecnum[e] = dd_to_double_int(pe);
   double f;
   if (o.tanh_form) {
-    f = 0.50 * (1.0 + tanh((dd_to_double(pe) - o.tanh_trans) / o.tanh_width));
+    f = 0.50 * (1.0 + tanh((dd_to_double_int(pe) - o.tanh_trans) / o.tanh_width));
   } else {
     const dd m = hf * pe;
     const dd m2 = m * m;
