@@ -994,10 +994,16 @@ __global__ void __launch_bounds__(kFusedChunk, kFusedPerSm)
   }
 }
 
-// applyDirichletBCs / resetRows: identity (or diag_value) rows. kResetLanes
-// lanes a row: one thread for a node's rows made one uncoalesced pass over its
-// entries, three rows of up to 18 on a hex wall (14 us for the walls of a box of 24x20x12 hexes, 2.6 now).
-constexpr int kResetLanes = 16;
+// applyDirichletBCs / resetRows: identity (or diag_value) rows, LANES lanes a row:
+// one thread for a node's rows made one uncoalesced pass over its entries, three
+// rows of up to 18 on a hex wall. Few or long rows take eight lanes, many short ones
+// four. With one thread a node, 16, 8 and 4 lanes a row (us, the host's wait
+// included): walls of 221 hex nodes, 3 unknowns, 28.7, 12.7, 12.7, 13.0; all rows of
+// 1.08 M hex nodes, 1 unknown (7 entries a row), 53.5, 148, 85, 51; with 3 unknowns
+// (21 entries) 801, 472, 288, 194; of 172,032 tet nodes with 3 unknowns (45 entries)
+// 276, 102, 73, 104.
+constexpr int64_t kResetFewRows = 4096;
+template <int LANES>
 __global__ void __launch_bounds__(kThreads)
     reset_rows_k(int64_t n, const int64_t* __restrict__ nodes,
                  const int64_t* __restrict__ node_lid, int num_dof,
@@ -1008,8 +1014,8 @@ __global__ void __launch_bounds__(kThreads)
                  const double* __restrict__ q,
                  const double* __restrict__ bc, int64_t num_nodes,
                  int* __restrict__ err) {
-  const int64_t t = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) / kResetLanes;
-  const int sub = int(threadIdx.x % kResetLanes), nd = max(end - begin, 1);
+  const int64_t t = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) / LANES;
+  const int sub = int(threadIdx.x % LANES), nd = max(end - begin, 1);
   const int64_t k = t / nd;
   if (k >= n) return;
   const int64_t node = nodes[k];
@@ -1021,7 +1027,7 @@ __global__ void __launch_bounds__(kThreads)
   const int d = begin + int(t - k * nd);
   const int64_t row = node_lid[node] + d;
   const int64_t p1 = row_ptr[row + 1];
-  for (int64_t p = row_ptr[row] + sub; p < p1; p += kResetLanes)
+  for (int64_t p = row_ptr[row] + sub; p < p1; p += LANES)
     values[p] = (col_idx[p] == row) ? diag_value : 0.0;
   if (sub == 0) rhs[row] = bc ? (bc[num_dof * node + d] - q[num_dof * node + d]) : rhs_value;
 }
@@ -1331,11 +1337,14 @@ void launch_reset_rows(cudaStream_t s, int64_t n, const int64_t* nodes,
                        int end, const int64_t* row_ptr, const int32_t* col_idx,
                        double* values, double* rhs, double diag_value,
                        double rhs_value, const double* q, const double* bc,
-                       int64_t num_nodes, int* err) {
+                       int64_t num_nodes, double row_length, int* err) {
   if (n == 0) return;
-  reset_rows_k<<<grid_for(n * std::max(end - begin, 1) * kResetLanes), kThreads, 0, s>>>(
-      n, nodes, node_lid, num_dof, begin, end, row_ptr, col_idx, values, rhs,
-      diag_value, rhs_value, q, bc, num_nodes, err);
+  const int64_t rows = n * std::max(end - begin, 1);
+  auto go = [&](auto kernel, int lanes) {
+    kernel<<<grid_for(rows * lanes), kThreads, 0, s>>>(n, nodes, node_lid, num_dof, begin, end, row_ptr, col_idx,
+                                                       values, rhs, diag_value, rhs_value, q, bc, num_nodes, err);
+  };
+  rows <= kResetFewRows || row_length >= 32.0 ? go(reset_rows_k<8>, 8) : go(reset_rows_k<4>, 4);
 }
 
 void launch_sum_into_block(cudaStream_t s, int n_ent, int num_dof,

@@ -92,7 +92,7 @@ void launch_reset_rows(cudaStream_t s, int64_t n, const int64_t* nodes,
                        int end, const int64_t* row_ptr, const int32_t* col_idx,
                        double* values, double* rhs, double diag_value,
                        double rhs_value, const double* q, const double* bc,
-                       int64_t num_nodes, int* err);
+                       int64_t num_nodes, double row_length, int* err);  // row_length: mean entries a row
 void launch_sum_into_block(cudaStream_t s, int n_ent, int num_dof,
                            const int64_t* ent_lid, const double* lhs,
                            const double* rhs_in, const int64_t* row_ptr,

@@ -741,7 +741,8 @@ nw_status nw_linsys_apply_dirichlet(nw_linsys* ls, int64_t n,
     materialize_zero(ls);
     launch_reset_rows(ls->stream, n, nodes, ls->node_lid.p, ls->num_dof, begin,
                       end, ls->row_ptr.p, ls->col_idx.p, ls->values.p,
-                      ls->rhs.p, 1.0, 0.0, q, bc, ls->g.num_nodes, ls->err);
+                      ls->rhs.p, 1.0, 0.0, q, bc, ls->g.num_nodes,
+                      double(ls->g.nnz) / double(ls->g.nrows), ls->err);
     NW_CUDA(cudaGetLastError());
     NW_CUDA(cudaStreamSynchronize(ls->stream));
     if (std::exchange(*ls->err, 0)) fail(NW_INVALID_ARG, "Dirichlet node index out of range");
@@ -760,7 +761,7 @@ nw_status nw_linsys_reset_rows(nw_linsys* ls, int64_t n, const int64_t* nodes,
     launch_reset_rows(ls->stream, n, nodes, ls->node_lid.p, ls->num_dof, begin,
                       end, ls->row_ptr.p, ls->col_idx.p, ls->values.p,
                       ls->rhs.p, diag_value, rhs_residual, nullptr, nullptr,
-                      ls->g.num_nodes, ls->err);
+                      ls->g.num_nodes, double(ls->g.nnz) / double(ls->g.nrows), ls->err);
     NW_CUDA(cudaGetLastError());
     NW_CUDA(cudaStreamSynchronize(ls->stream));
     if (std::exchange(*ls->err, 0)) fail(NW_INVALID_ARG, "resetRows node index out of range");
