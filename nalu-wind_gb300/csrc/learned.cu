@@ -222,15 +222,18 @@ __global__ void colsum_k(int nblocks, int ncols, const float* __restrict__ parti
   dst[j] = accumulate ? dst[j] + s : s;
 }
 
-constexpr int kAggBatch = 32;  // gathers in flight
+constexpr int kAggBatch = 8;  // gathers in flight
 
 // ---------------------------------------------------------------------------
 // Aggregation over the coarse graph (diagonal slot skipped):
 // out[I][64 + c] = sum_J w_IJ in[J][c], in/out BF16 with row stride 128.
-// Bound by the latency of the gathered rows: the lanes load a row's columns
-// and weights together and up to 32 gathers are in flight, then the
-// multiply-adds in column order: 1,216 rows take 3.8 us, 5.0 with one load,
-// gather and multiply-add after the other.
+// Bound by the latency of the gathered rows, and by the warps in flight where
+// there are many rows: the lanes load a row's columns and weights together and
+// eight gathers are in flight, then the multiply-adds in column order. An
+// iteration of the learned solve with 4, 8, 16 and 32 gathers: 321,489 unknowns
+// 102.8, 93.2, 93.3, 94.6 us; 2.1 M 293, 285, 288, 297; 8.5 M 1,017, 992, 1,002,
+// 1,039 (this kernel, 29,248 rows: 39.6 us with 32, 19.0 with one load, gather and
+// multiply-add after the other, 17.8 now).
 __global__ void __launch_bounds__(kB)
     agg_fwd_k(int64_t nc, const int64_t* __restrict__ cptr,
               const int32_t* __restrict__ ccol, const int32_t* __restrict__ cdiag,
