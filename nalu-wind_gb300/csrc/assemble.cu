@@ -103,7 +103,7 @@ __device__ __forceinline__ void ld32(const double* p, double (&x)[4]) {
 // takes one reciprocal for both of its divisions, the tanh form 0.5 (1 +
 // tanh x) is 1 / (1 + exp(-2 x)), and with alpha = 0 (the default) only the
 // upwind side is extrapolated and limited. 68 FP64 instructions an edge
-// against 132 (classic), 105 against 196 (limiter and tanh): 476,280 nodes
+// against 132 (classic), 104 against 196 (limiter and tanh): 476,280 nodes
 // 576 -> 333 us with the row phase. Errors of the entries against extended
 // precision (rms, 49 x 40 x 30 hexes, tanh and relax 0.7; 132 and 196
 // instructions and now): downwind side 1.88e-16 and 1.59e-16, upwind side
